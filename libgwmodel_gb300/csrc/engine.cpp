@@ -597,8 +597,8 @@ bool Engine::hatUpdateFx(double bw, bool adaptive, int kernel, const double* T, 
     }
     hat_exp_.alloc((size_t)((n_ + 1023) / 1024) * groups * 64);
     hat_state_.alloc(1);
-    check(launch_build_zfx(n_, n_, 64, groups, T, n_, x_.get(), hat_img_.get(), hat_exp_.get(), hat_state_.get(),
-                           stream_),
+    check(launch_build_zfx(n_, n_, 64, groups, T, n_, x_.get(), hat_img_.get(), hat_exp_.get(), nullptr,
+                           hat_state_.get(), stream_),
           "build_zfx");
     FxArgs a = fxArgs(bw, adaptive ? thr_.get() : nullptr);
     setFocus(a, fxFocus(), tb16_.get(), n_, true);
@@ -622,7 +622,7 @@ bool Engine::hatUpdateFx(double bw, bool adaptive, int kernel, const double* T, 
 void Engine::synchronizeFx()
 {
     if (zfx_ready_)
-        check(cudaMemcpyAsync(host_sums_ + 6, fx_state_.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
+        check(cudaMemcpyAsync(host_sums_ + 6, fx_state_.get(), 3 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
     synchronize();
     if (zfx_ready_) fxCheck();
 }
@@ -1133,20 +1133,23 @@ bool Engine::buildZfx(bool mixed)
     const int tiles = (n_ + kTile - 1) / kTile;
     zfx_n_ = fx_columns(m_, &zfx_groups_);
     zfx_.alloc((size_t)tiles * zfx_groups_ * zfx_n_ * 256);
-    zfx_exp_.alloc((size_t)((n_ + 1023) / 1024) * zfx_groups_ * zfx_n_);
+    const size_t scales = (size_t)((n_ + 1023) / 1024) * zfx_groups_ * zfx_n_;
+    zfx_exp_.alloc(scales);
+    zfx_sum_.alloc(2 * scales);
+    fx_lim_.alloc(2 * (size_t)p_);
     if (!fx_state_.get()) {
-        fx_state_.alloc(2);
-        check(cudaMemsetAsync(fx_state_.get(), 0, 2 * sizeof(int), stream_), "memset");
+        fx_state_.alloc(3);
+        check(cudaMemsetAsync(fx_state_.get(), 0, 3 * sizeof(int), stream_), "memset");
     }
     check(launch_build_zfx(n_, m_, zfx_n_, zfx_groups_, mixed ? zs_.get() : z_.get(), m_, nullptr, zfx_.get(),
-                           zfx_exp_.get(), fx_state_.get(), stream_),
+                           zfx_exp_.get(), zfx_sum_.get(), fx_state_.get(), stream_),
           "build_zfx");
     stats_.kernel_launches += 1;
     zfx_ready_ = true;
     zfx_kind_ = mixed ? 2 : 1;
     zfx_bad_ = -1;
     if (mixed) {  // the caller has no FP64 sums to fall back on in the same stream: ask now, once per X and y
-        check(cudaMemcpyAsync(host_sums_ + 6, fx_state_.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
+        check(cudaMemcpyAsync(host_sums_ + 6, fx_state_.get(), 3 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
         synchronize();
         fxCheck();
     }
@@ -1254,7 +1257,7 @@ bool Engine::scratchFits(size_t bytes, size_t held) const
 
 bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcols, double* G, int ldg,
                         const double* thr, double bw, int kernel, bool exclude_self, int wpow, bool exact,
-                        WeightUse use)
+                        double points, WeightUse use)
 {
     const bool flags = exclude_self || focus != fxFocus() || !exact || zfx_bad_ < 0;
     FxArgs a = fxArgs(bw, thr);
@@ -1267,6 +1270,12 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
     a.zimg = zfx_.get();
     a.zexp = zfx_exp_.get();
     a.zcols = zfx_n_ * zfx_groups_;
+    a.limits.p = p_;
+    a.limits.points = points;
+    a.limits.root = std::sqrt(points);
+    a.limits.zsum = zfx_sum_.get();
+    a.limits.off = fx_state_.get();
+    a.limits.lim = fx_lim_.get() + (wpow == 2 ? p_ : 0);
     const int groups = (mcols + zfx_n_ - 1) / zfx_n_;
     // Further column groups and passes read the first group's weights back: making them
     // takes some 10 times as long as the rest of a tile (n = 20,011, p = 17, great-circle).
@@ -1313,13 +1322,51 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
 
 void Engine::fxCheck()
 {
-    int st[2];
+    int st[3];
     std::memcpy(st, host_sums_ + 6, sizeof(st));
     zfx_bad_ = st[0] != 0;
-    if (st[1]) {
-        check(cudaMemsetAsync(fx_state_.get() + 1, 0, sizeof(int), stream_), "memset");
+    guard_hit_ = guard_hit_ || st[2] != 0;
+    if (st[1] || st[2]) {
+        check(cudaMemsetAsync(fx_state_.get() + 1, 0, 2 * sizeof(int), stream_), "memset");
         synchronize();
-        throw CudaError("fixed-point contraction: a bounded wait timed out");
+    }
+    if (st[1]) throw CudaError("fixed-point contraction: a bounded wait timed out");
+}
+
+// Points that can have weight at a row: an adaptive threshold of a compact kernel leaves
+// it to the neighbours it counts.
+double Engine::fxPoints(double bw, bool adaptive, int kernel) const
+{
+    return adaptive && kernel >= GW_KERNEL_BISQUARE ? std::min((double)n_, bw + 1.0) : (double)n_;
+}
+
+FxGuard Engine::fxGuard(int rows, const int* done)
+{
+    const int blocks = (rows + kRowBlock - 1) / kRowBlock;
+    if (guard_hit_ || (int)guard_flags_.size() != blocks) {  // otherwise no block is marked
+        guard_flags_.alloc(blocks);
+        check(cudaMemsetAsync(guard_flags_.get(), 0, sizeof(int) * blocks, stream_), "memset");
+        guard_hit_ = false;
+    }
+    FxGuard g{};
+    g.lim = fx_lim_.get();
+    g.done = done;
+    g.flags = guard_flags_.get();
+    g.any = fx_state_.get() + 2;
+    return g;
+}
+
+// The FP64 contraction over every row block, or only those that flags marks unless *all.
+void Engine::contractRows(const double* Z, int mcols, double* G, int ldg, double bw, bool adaptive, int kernel,
+                          bool exclude_self, int wpow, const int* flags, const int* all)
+{
+    // the kernel takes at most 256 columns (p <= 21); wider Z (p up to 32) in column chunks
+    for (int c0 = 0; c0 < mcols; c0 += 256) {
+        const int w = std::min(256, mcols - c0);
+        check(launch_contract64(points(), geographic_, tb16_.get(), Z + c0, m_, w, G + c0, ldg, thrPtr(adaptive), bw,
+                                kernel, exclude_self, wpow, true, stream_, flags, all),
+              "contract64");
+        stats_.kernel_launches += 1;
     }
 }
 
@@ -1327,18 +1374,19 @@ void Engine::contract(const double* Z, int mcols, double* G, int ldg, double bw,
                       bool exclude_self, int wpow, WeightUse use)
 {
     cudaEvent_t e0 = stats_on_ ? timerBegin() : nullptr;
-    // the kernel takes at most 256 columns (p <= 21); wider Z (p up to 32) in column chunks
     const bool fx = fxReady(kernel);
     if (use != WeightUse::kAgain) fx_weights_kept_ = false;
     const bool rest = !fx || contractFx(fxFocus(), tb16_.get(), n_, mcols, G, ldg, thrPtr(adaptive), bw, kernel,
-                                        exclude_self, wpow, ixy_exact_, use);
-    for (int c0 = 0; rest && c0 < mcols; c0 += 256) {
-        const int w = std::min(256, mcols - c0);
-        check(launch_contract64(points(), geographic_, tb16_.get(), Z + c0, m_, w, G + c0, ldg, thrPtr(adaptive), bw,
-                                kernel, exclude_self, wpow, true, stream_, fx ? fx_flags_.get() : nullptr,
-                                fx ? fx_state_.get() : nullptr),
-              "contract64");
-        stats_.kernel_launches += 1;
+                                        exclude_self, wpow, ixy_exact_, fxPoints(bw, adaptive, kernel), use);
+    if (rest)
+        contractRows(Z, mcols, G, ldg, bw, adaptive, kernel, exclude_self, wpow, fx ? fx_flags_.get() : nullptr,
+                     fx ? fx_state_.get() : nullptr);
+    if (wpow == 1) {
+        g_fx_ = fx;
+        g_flagged_ = fx && rest;
+        g2_fx_ = false;
+    } else {
+        g2_fx_ = fx;
     }
     if (stats_on_) {
         timerEnd(e0, 0);
@@ -1398,9 +1446,26 @@ void Engine::solve(int mode, double bw, bool adaptive, int kernel, double out[4]
     const bool fx = zfx_ready_;
     a.out = criterionOut();
     if (mixed) a.out.err = err_.get();
+    const bool guarded = !mixed && g_fx_ && zfx_bad_ != 1;
+    if (guarded) {
+        // (a second pass has its own flags: its blocks are tested whatever the first one's hold)
+        a.guard = fxGuard(n_, g_flagged_ && !g2_fx_ ? fx_flags_.get() : nullptr);
+        if (mode == kSolveFit && g2_fx_) a.guard.lim2 = fx_lim_.get() + p_;
+    }
     check(launch_solve(a, &nb, stream_), "solve");
     synchronize();
     if (fx) fxCheck();
+    if (guarded && guard_hit_) {
+        contractRows(z_.get(), m_, g_.get(), m_, bw, adaptive, kernel, mode == kSolveCV, 1, guard_flags_.get(),
+                     fx_state_.get());
+        if (a.guard.lim2)
+            contractRows(z_.get(), mm_, g2_.get(), mm_, bw, adaptive, kernel, false, 2, guard_flags_.get(),
+                         fx_state_.get());
+        a.guard = FxGuard{};
+        check(launch_solve(a, &nb, stream_), "solve");
+        stats_.kernel_launches += 1;
+        synchronize();
+    }
     for (int q = 0; q < 4; q++) out[q] = host_sums_[q];
     {
         int serr = 0;
@@ -1790,22 +1855,27 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     // X^T W_i X, X^T W_i y at every location, then beta_i = (X^T W_i X)^-1 X^T W_i y
     pf_g_.alloc((size_t)nr * m_);
     bool fx = fxReady(kernel), fexact = ixy_exact_;
+    const double reached = fxPoints(bw, adaptive, kernel);
     if (fx && geographic_ && withinCap(fe)) {
         pf_ie3_.alloc(nr);
         check(launch_int_vectors(nr, pf_uR_.get(), pf_vR_.get(), pf_ie3_.get(), stream_), "integer unit vectors");
-        contractFx(pf_ie3_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, true);
+        contractFx(pf_ie3_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, true, reached);
     } else if (fx && !geographic_ && integerCoords(nr, pf_u_.get(), pf_v_.get(), pf_ixy_, fexact)) {
-        contractFx(pf_ixy_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, fexact);
+        contractFx(pf_ixy_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, fexact,
+                   reached);
     } else {
         fx = false;
     }
-    for (int c0 = 0; c0 < m_; c0 += 256) {  // at most 256 columns a launch
-        check(launch_contract64_focus(points(), tb16_.get(), F, pf_tb16_.get(), geographic_, z_.get() + c0, m_,
-                                      std::min(256, m_ - c0), pf_g_.get() + c0, m_, thr, bw, kernel, false, 1, true,
-                                      stream_, fx ? fx_flags_.get() : nullptr, fx ? fx_state_.get() : nullptr),
-              "predict contraction");
-        stats_.kernel_launches += 1;
-    }
+    const auto contractFocus = [&](const int* flags) {
+        for (int c0 = 0; c0 < m_; c0 += 256) {  // at most 256 columns a launch
+            check(launch_contract64_focus(points(), tb16_.get(), F, pf_tb16_.get(), geographic_, z_.get() + c0, m_,
+                                          std::min(256, m_ - c0), pf_g_.get() + c0, m_, thr, bw, kernel, false, 1, true,
+                                          stream_, flags, flags ? fx_state_.get() : nullptr),
+                  "predict contraction");
+            stats_.kernel_launches += 1;
+        }
+    };
+    contractFocus(fx ? fx_flags_.get() : nullptr);
     pf_beta_.alloc((size_t)nr * p);
     SolveArgs a{};
     a.n = nr;
@@ -1822,8 +1892,7 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     int nb = 0;
     a.out = criterionOut();
     if (!fx) a.out.fx_state = nullptr;
-    check(launch_solve(a, &nb, stream_), "predict solve");
-    stats_.kernel_launches += 3;
+    if (fx) a.guard = fxGuard(nr, fx_flags_.get());
     UnpermuteArgs un{};
     un.n = nr;
     un.perm = pf_perm_.get();
@@ -1831,12 +1900,24 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     un.src[0] = pf_beta_.get();
     out_.alloc((size_t)nr * p);
     un.dst[0] = out_.get();
-    check(launch_unpermute(un, 1, stream_), "unpermute");
-    stats_.kernel_launches += 1;
     betas.resize((size_t)nr * p);
-    check(cudaMemcpyAsync(betas.data(), out_.get(), sizeof(double) * betas.size(), cudaMemcpyDeviceToHost, stream_), "D2H");
-    synchronize();
-    if (fx) fxCheck();
+    const auto solveAll = [&] {
+        check(launch_solve(a, &nb, stream_), "predict solve");
+        check(launch_unpermute(un, 1, stream_), "unpermute");
+        stats_.kernel_launches += 4;
+        check(cudaMemcpyAsync(betas.data(), out_.get(), sizeof(double) * betas.size(), cudaMemcpyDeviceToHost, stream_),
+              "D2H");
+        synchronize();
+    };
+    solveAll();
+    if (fx) {
+        fxCheck();
+        if (guard_hit_) {
+            contractFocus(guard_flags_.get());
+            a.guard = FxGuard{};
+            solveAll();
+        }
+    }
     int serr = 0;
     std::memcpy(&serr, host_sums_ + 5, sizeof(int));
     if (serr) throw CudaError("adaptive threshold select failed (code " + std::to_string(serr) + ")");

@@ -296,7 +296,7 @@ private:
     bool integerCoords(int n, const double* u, const double* v, DevBuf<longlong2>& out, bool& exact);
     bool withinCap(const std::vector<double>& e) const;
     bool contractFx(const void* focus, const float4* ftb16, int nf, int mcols, double* G, int ldg, const double* thr,
-                    double bw, int kernel, bool exclude_self, int wpow, bool exact,
+                    double bw, int kernel, bool exclude_self, int wpow, bool exact, double points,
                     WeightUse use = WeightUse::kOnce);
     FxMode fxMode(int kernel) const;
     FxArgs fxArgs(double bw, const double* thr) const;
@@ -315,12 +315,23 @@ private:
     bool refineFx(double bw, bool adaptive, int kernel, const float* d2c);
     int zfx_kind_ = 0;          // whose images zfx_ holds: 1 z_, 2 zs_
     void fxCheck();  // after a synchronisation that copied fx_state_ to host_sums_ + 6
+    // Rows whose fixed-point sums the solve finds less exact than FP64 ones (FxGuard), by
+    // 64-row blocks: recomputed in FP64 (contractRows) and solved again.
+    FxGuard fxGuard(int rows, const int* done);
+    double fxPoints(double bw, bool adaptive, int kernel) const;
+    void contractRows(const double* Z, int mcols, double* G, int ldg, double bw, bool adaptive, int kernel,
+                      bool exclude_self, int wpow, const int* flags, const int* all);
+    DevBuf<double> zfx_sum_, fx_lim_;  // fx_lim_: limits of G, then of G2
+    DevBuf<int> guard_flags_;
+    bool guard_hit_ = false;             // guard_flags_ marks rows of the last guarded solve
+    bool g_fx_ = false, g2_fx_ = false;  // g_, g2_ hold fixed-point sums
+    bool g_flagged_ = false;             // ... whose blocks in fx_flags_ k_contract64 has recomputed
     DevBuf<longlong2> ixy_, pf_ixy_;
     int iscale_ = 0;
     double iu0_ = 0.0, iv0_ = 0.0;
     bool ixy_tried_ = false, ixy_ok_ = false, ixy_exact_ = false;
     DevBuf<unsigned char> zfx_;
-    DevBuf<int> zfx_exp_, fx_state_, fx_flags_;  // fx_state_: {Z unsuitable, wait timed out}
+    DevBuf<int> zfx_exp_, fx_state_, fx_flags_;  // fx_state_: {Z unsuitable, wait timed out, guard_flags_ marks rows}
     DevBuf<double> fx_part_;
     DevBuf<unsigned> fx_rowmax_;
     bool zfx_ready_ = false;

@@ -123,6 +123,33 @@ cudaError_t launch_contract64_focus(const DevPoints& P, const float4* tb16, cons
                                     bool skip_tiles, cudaStream_t stream, const int* flags = nullptr,
                                     const int* all = nullptr);
 
+// Which rows of fixed-point sums are less exact than FP64 ones because a column of X
+// rests on small weights there (a covariate that is zero near the row's location): the
+// sums' errors are absolute, so the diagonals G_kk tell.  A row is low when G_kk of a
+// column is below
+//     lim_k = max(2^-17 T_k, 2^-14 V_k),  V_k = sqrt(sum_j 4^e_jk),
+// T_k = sum_j x_jk^2 (truncated weights: 2^-60 T_k at most) and e_jk the exponent of the
+// scale of each nonzero x_jk^2 (dropped digits: 2^-62 V_k, root mean square); 2^-14 T_k for
+// squared weights.  Off-diagonal errors follow by Cauchy's inequality.  Measured against
+// long double sums (2,000 and 10,000 points, an indicator or a lognormal column, gaussian
+// and bisquare): above these lines coefficients are at most 1.1e-15 off and squared sums
+// 1.2e-15, FP64 weights 2.3e-15 and 2.6e-15; at 2^-20 to 2^-25 they are 3e-14 and 3e-12 off.
+// T_k and V_k count at most `points` points of the largest value (a compact kernel's
+// neighbours).  The limits come with the sums (launch_contract_fx); the solve, which
+// reads every G_kk anyway, tests them: flags[row / 64] and *any are set.
+struct FxLimits {
+    int p;               // columns of X
+    double points, root; // and its square root
+    const double* zsum;  // launch_build_zfx's
+    const int* off;      // nonzero: FP64 sums follow, every limit is 0
+    double* lim;         // p limits; null: none wanted
+};
+struct FxGuard {
+    const double *lim, *lim2;  // limits of G and, optional, of G2 (fit mode); null: no test
+    const int* done;           // optional: 64-row blocks that hold FP64 sums already
+    int *flags, *any;
+};
+
 // The same sums on the tensor cores, in 62-bit fixed point (k_contract_fx.cu):
 // bisquare and gaussian weights; geographic points within one spherical cap of
 // chord radius 1/2.
@@ -159,6 +186,7 @@ struct FxArgs {
     // tile x 16 points x 128 rows (fx_weight_bytes); wstore writes them, wload reads them.
     unsigned long long* wstore;
     const unsigned long long* wload;
+    FxLimits limits;
 };
 // Bytes of the kept weights of nf rows and n points.
 size_t fx_weight_bytes(int nf, int n);
@@ -170,9 +198,10 @@ int fx_splits(int blocks, int ntiles, int num_sms);
 cudaError_t launch_int_vectors(int n, const double* lon, const double* lat, fx::Vec3* out, cudaStream_t stream);
 // img: (n / 16 tiles rounded up) x groups x N x 256 bytes; zexp: scale blocks of
 // 1024 points x (N groups); *bad: whether Z needs FP64 sums instead.  With x the
-// operand is x_j (Z[j, c] + [j = c]) (the multiscale hat update).
+// operand is x_j (Z[j, c] + [j = c]) (the multiscale hat update).  zsum (null with x): per
+// entry of zexp the sum of |Z| and the number of nonzeros.
 cudaError_t launch_build_zfx(int n, int ncols, int N, int groups, const double* Z, int ldz, const double* x,
-                             unsigned char* img, int* zexp, int* bad, cudaStream_t stream);
+                             unsigned char* img, int* zexp, double* zsum, int* bad, cudaStream_t stream);
 // r = b - A beta of every row's packed normal equations (n x p).
 cudaError_t launch_normal_residual(int n, int p, const double* G, int ldg, const double* beta, double* r,
                                    cudaStream_t stream);
@@ -187,11 +216,11 @@ cudaError_t launch_fx_finish(const FxArgs& a, int nsplit, double* G, int ldg, in
 //
 // Where the sums go when the caller waits for them: pinned host memory, written by the
 // kernel that forms them (host[0 .. 3] the sums, then as integers host[4] = *err,
-// host[5] = *sel_err, host[6] = fx_state[0 .. 1]; null sources are left out).  A copy per
+// host[5] = *sel_err, host[6 .. 7] = fx_state[0 .. 2]; null sources are left out).  A copy per
 // value cost about 2.5 us each on the stream.  ticket: a zeroed counter, zero again afterwards.
 struct CriterionOut {
     double* host;
-    const int *err, *sel_err, *fx_state;
+    const int *err, *sel_err, *fx_state;  // fx_state: three words
     unsigned* ticket;
 };
 struct SolveArgs {
@@ -221,6 +250,7 @@ struct SolveArgs {
     double* ainv;
     // launch_solve, optional: the partial blocks are summed too (as launch_reduce_partials)
     CriterionOut out;
+    FxGuard guard;
 };
 // Largest grid launch_solve uses; callers size `partials` (4 doubles per block) for it.
 constexpr int kSolveMaxBlocks = 4096;
