@@ -530,7 +530,8 @@ void Engine::hatPass(double bw, bool adaptive, int kernel, double* S, int row_ta
     a.thr = thrPtr(adaptive);
     a.bw = bw;
     a.kernel = kernel;
-    if (fxReady(kernel) && ixy_exact_) {
+    // v_i = A_i^-1 x_i is large where a column rests on small weights: FP64 ones there too
+    if (fxReady(kernel) && ixy_exact_ && !guard_hit_) {
         hat_rows_.alloc(n_);
         a.xy = geographic_ ? nullptr : ixy_.get();
         a.e3 = geographic_ ? ie3_.get() : nullptr;

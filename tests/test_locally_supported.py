@@ -75,3 +75,19 @@ def test_indicator_among_many_columns(p):
     rng = np.random.default_rng(p)
     x = np.asfortranarray(np.column_stack([x, rng.standard_normal((n, p - 3))]))
     check(engine(x, y, c, False), O.Problem(x, y, c), 9.0 if p == 11 else 14.0, False, O.GAUSSIAN)
+
+
+@pytest.mark.parametrize("geographic", [False, True])
+@pytest.mark.parametrize("kernel,bw,store", [(O.GAUSSIAN, 6.0, False), (O.GAUSSIAN, 9.0, False), (O.BISQUARE, None, True)])
+def test_hat_matrix_of_an_indicator(kernel, bw, store, geographic):
+    """s_ij = w_ij v_i . x_j with v_i = A_i^-1 x_i as large as the column's weights are small: qDiag and S."""
+    n = 600
+    x, y, c = problem(n, 4, geographic)
+    e, ref = engine(x, y, c, geographic), O.Problem(x, y, c, geographic=geographic)
+    bw = bw * (10.0 if geographic else 1.0) if bw else 1.002 * max(ref.distance_row(i)[x[:, 2] > 0].min() for i in range(n))
+    want = ref.fit_core(bw, False, kernel, True)
+    for repeat in range(2):
+        got = e.fit(bw, False, kernel, store)
+        np.testing.assert_allclose(got[3], want[3], rtol=1e-9)
+        if store:
+            assert np.abs(got[4] - want[4]).max() <= 1e-9 * np.abs(want[4]).max()
