@@ -1184,6 +1184,7 @@ bool Engine::refineFx(double bw, bool adaptive, int kernel, const float* d2c)
     a.zexp = zfx_exp_.get();
     a.zcols = zfx_n_ * zfx_groups_;
     a.err = fx_state_.get() + 1;
+    a.limits = fxLimits(bw, adaptive, kernel, 1);
     // the contraction's sums are free by now: rows of at most npad doubles
     double* G = reinterpret_cast<double*>(acc_.get());
     const int nsplit = fx_splits((n_ + 127) / 128 * zfx_groups_, tiles, num_sms_);
@@ -1198,8 +1199,10 @@ bool Engine::refineFx(double bw, bool adaptive, int kernel, const float* d2c)
     }
     check(launch_contract_fx(a, geographic_ ? kFxMixedGeo : kFxMixed, nsplit, stream_), "contract_fx");
     check(launch_fx_finish(a, nsplit, G, m_, nullptr, stream_), "fx_finish");
-    check(launch_normal_residual(n_, p_, G, m_, beta_.get(), rvec_.get(), stream_), "residual");
-    stats_.kernel_launches += nsplit > 1 ? 2 : 1;
+    refine_low_.alloc((n_ + kResidualRows - 1) / kResidualRows);
+    check(launch_normal_residual(n_, p_, G, m_, beta_.get(), fx_lim_.get(), rvec_.get(), refine_low_.get(), stream_),
+          "residual");
+    stats_.kernel_launches += nsplit > 1 ? 3 : 2;
     return true;
 }
 
@@ -1258,7 +1261,7 @@ bool Engine::scratchFits(size_t bytes, size_t held) const
 
 bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcols, double* G, int ldg,
                         const double* thr, double bw, int kernel, bool exclude_self, int wpow, bool exact,
-                        double points, WeightUse use)
+                        const FxLimits& limits, WeightUse use)
 {
     const bool flags = exclude_self || focus != fxFocus() || !exact || zfx_bad_ < 0;
     FxArgs a = fxArgs(bw, thr);
@@ -1271,12 +1274,7 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
     a.zimg = zfx_.get();
     a.zexp = zfx_exp_.get();
     a.zcols = zfx_n_ * zfx_groups_;
-    a.limits.p = p_;
-    a.limits.points = points;
-    a.limits.root = std::sqrt(points);
-    a.limits.zsum = zfx_sum_.get();
-    a.limits.off = fx_state_.get();
-    a.limits.lim = fx_lim_.get() + (wpow == 2 ? p_ : 0);
+    a.limits = limits;
     const int groups = (mcols + zfx_n_ - 1) / zfx_n_;
     // Further column groups and passes read the first group's weights back: making them
     // takes some 10 times as long as the rest of a tile (n = 20,011, p = 17, great-circle).
@@ -1334,11 +1332,17 @@ void Engine::fxCheck()
     if (st[1]) throw CudaError("fixed-point contraction: a bounded wait timed out");
 }
 
-// Points that can have weight at a row: an adaptive threshold of a compact kernel leaves
-// it to the neighbours it counts.
-double Engine::fxPoints(double bw, bool adaptive, int kernel) const
+FxLimits Engine::fxLimits(double bw, bool adaptive, int kernel, int wpow) const
 {
-    return adaptive && kernel >= GW_KERNEL_BISQUARE ? std::min((double)n_, bw + 1.0) : (double)n_;
+    FxLimits l{};
+    l.p = p_;
+    // an adaptive threshold of a compact kernel leaves weight to the neighbours it counts
+    l.points = adaptive && kernel >= GW_KERNEL_BISQUARE ? std::min((double)n_, bw + 1.0) : (double)n_;
+    l.root = std::sqrt(l.points);
+    l.zsum = zfx_sum_.get();
+    l.off = fx_state_.get();
+    l.lim = fx_lim_.get() + (wpow == 2 ? p_ : 0);
+    return l;
 }
 
 FxGuard Engine::fxGuard(int rows, const int* done)
@@ -1378,7 +1382,8 @@ void Engine::contract(const double* Z, int mcols, double* G, int ldg, double bw,
     const bool fx = fxReady(kernel);
     if (use != WeightUse::kAgain) fx_weights_kept_ = false;
     const bool rest = !fx || contractFx(fxFocus(), tb16_.get(), n_, mcols, G, ldg, thrPtr(adaptive), bw, kernel,
-                                        exclude_self, wpow, ixy_exact_, fxPoints(bw, adaptive, kernel), use);
+                                        exclude_self, wpow, ixy_exact_,
+                                        fxLimits(bw, adaptive, kernel, wpow), use);
     if (rest)
         contractRows(Z, mcols, G, ldg, bw, adaptive, kernel, exclude_self, wpow, fx ? fx_flags_.get() : nullptr,
                      fx ? fx_state_.get() : nullptr);
@@ -1512,8 +1517,10 @@ void Engine::refine(double bw, bool adaptive, int kernel, double out[4])
         r.d2c = ensureDistanceCache();
         if (!r.d2c) d2lock.unlock();
     }
-    if (!refineFx((float)bw, adaptive, kernel, r.d2c))
-        check(launch_refine_residual(r, geographic_, stream_), "refine residual");
+    // the residuals that the fixed-point sums give, but of rows where a column rests on
+    // weights near 2^-62 (FxLimits), which the double-float pass holds in full
+    if (refineFx((float)bw, adaptive, kernel, r.d2c)) r.low = refine_low_.get();
+    check(launch_refine_residual(r, geographic_, stream_), "refine residual");
     stats_.kernel_launches += 1;
     if (r.d2c) {
         check(cudaEventRecord(dc.used, stream_), "cudaEventRecord");
@@ -1856,14 +1863,15 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     // X^T W_i X, X^T W_i y at every location, then beta_i = (X^T W_i X)^-1 X^T W_i y
     pf_g_.alloc((size_t)nr * m_);
     bool fx = fxReady(kernel), fexact = ixy_exact_;
-    const double reached = fxPoints(bw, adaptive, kernel);
+    FxLimits limits{};
+    if (fx) limits = fxLimits(bw, adaptive, kernel, 1);
     if (fx && geographic_ && withinCap(fe)) {
         pf_ie3_.alloc(nr);
         check(launch_int_vectors(nr, pf_uR_.get(), pf_vR_.get(), pf_ie3_.get(), stream_), "integer unit vectors");
-        contractFx(pf_ie3_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, true, reached);
+        contractFx(pf_ie3_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, true, limits);
     } else if (fx && !geographic_ && integerCoords(nr, pf_u_.get(), pf_v_.get(), pf_ixy_, fexact)) {
         contractFx(pf_ixy_.get(), pf_tb16_.get(), nr, m_, pf_g_.get(), m_, thr, bw, kernel, false, 1, fexact,
-                   reached);
+                   limits);
     } else {
         fx = false;
     }

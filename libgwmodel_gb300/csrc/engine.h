@@ -296,7 +296,7 @@ private:
     bool integerCoords(int n, const double* u, const double* v, DevBuf<longlong2>& out, bool& exact);
     bool withinCap(const std::vector<double>& e) const;
     bool contractFx(const void* focus, const float4* ftb16, int nf, int mcols, double* G, int ldg, const double* thr,
-                    double bw, int kernel, bool exclude_self, int wpow, bool exact, double points,
+                    double bw, int kernel, bool exclude_self, int wpow, bool exact, const FxLimits& limits,
                     WeightUse use = WeightUse::kOnce);
     FxMode fxMode(int kernel) const;
     FxArgs fxArgs(double bw, const double* thr) const;
@@ -318,7 +318,8 @@ private:
     // Rows whose fixed-point sums the solve finds less exact than FP64 ones (FxGuard), by
     // 64-row blocks: recomputed in FP64 (contractRows) and solved again.
     FxGuard fxGuard(int rows, const int* done);
-    double fxPoints(double bw, bool adaptive, int kernel) const;
+    FxLimits fxLimits(double bw, bool adaptive, int kernel, int wpow) const;
+    DevBuf<int> refine_low_;
     void contractRows(const double* Z, int mcols, double* G, int ldg, double bw, bool adaptive, int kernel,
                       bool exclude_self, int wpow, const int* flags, const int* all);
     DevBuf<double> zfx_sum_, fx_lim_;  // fx_lim_: limits of G, then of G2

@@ -202,9 +202,11 @@ cudaError_t launch_int_vectors(int n, const double* lon, const double* lat, fx::
 // entry of zexp the sum of |Z| and the number of nonzeros.
 cudaError_t launch_build_zfx(int n, int ncols, int N, int groups, const double* Z, int ldz, const double* x,
                              unsigned char* img, int* zexp, double* zsum, int* bad, cudaStream_t stream);
-// r = b - A beta of every row's packed normal equations (n x p).
-cudaError_t launch_normal_residual(int n, int p, const double* G, int ldg, const double* beta, double* r,
-                                   cudaStream_t stream);
+// r = b - A beta of every row's packed normal equations (n x p), and for each kResidualRows
+// rows in low[] whether a diagonal is below its limit (FxLimits::lim).
+constexpr int kResidualRows = 8;
+cudaError_t launch_normal_residual(int n, int p, const double* G, int ldg, const double* beta, const double* lim,
+                                   double* r, int* low, cudaStream_t stream);
 cudaError_t launch_contract_fx(const FxArgs& a, int mode, int nsplit, cudaStream_t stream);
 // Sums the splits into G and, with flags, marks the 64-row blocks that need FP64 sums.
 cudaError_t launch_fx_finish(const FxArgs& a, int nsplit, double* G, int ldg, int* flags, cudaStream_t stream);
@@ -393,6 +395,7 @@ struct RefineArgs {
     float bw;
     double* r;            // n x p
     const float* d2c;     // geographic only, optional: the distance cache (the contraction's FP32 d^2)
+    const int* low;       // optional: only the 128-row blocks with a mark of launch_normal_residual
 };
 cudaError_t launch_refine_residual(const RefineArgs& a, bool geographic, cudaStream_t stream);
 

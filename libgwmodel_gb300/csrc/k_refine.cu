@@ -83,6 +83,9 @@ __global__ void __launch_bounds__(RF_THREADS) k_refine(RefineArgs a)
     const int row0 = blockIdx.x * RF_THREADS;
     const int i = row0 + t;
     const bool ok = i < a.n;
+    if (a.low && !__syncthreads_or(t < RF_THREADS / kResidualRows && row0 + t * kResidualRows < a.n &&
+                                   a.low[row0 / kResidualRows + t]))
+        return;
 
     float4 fa = make_float4(0.f, 0.f, 0.f, 0.f), fb = fa;
     if (ok) {
