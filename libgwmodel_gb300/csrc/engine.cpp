@@ -586,7 +586,9 @@ void Engine::hatUpdate(double bw, bool adaptive, int kernel, const double* T, do
 // tells that T is not finite.
 bool Engine::hatUpdateFx(double bw, bool adaptive, int kernel, const double* T, double* SA)
 {
-    if (!fxReady(kernel) || !ixy_exact_) return false;
+    // v_i is as large as the variable's weights near i are small, if x_i is not 0 (then the
+    // row is 0): weights below 2^-62 would be missing from s_ij = v_i w_ij x_j up to 2^-32
+    if (!fxReady(kernel) || !ixy_exact_ || (guard_hit_ & 2)) return false;
     const int tiles = (n_ + kTile - 1) / kTile, groups = (n_ + 63) / 64;
     const size_t bytes = (size_t)tiles * groups * 64 * 256;
     if (!fx_fits(64, tiles)) return false;
@@ -1324,7 +1326,7 @@ void Engine::fxCheck()
     int st[3];
     std::memcpy(st, host_sums_ + 6, sizeof(st));
     zfx_bad_ = st[0] != 0;
-    guard_hit_ = guard_hit_ || st[2] != 0;
+    guard_hit_ |= st[2];
     if (st[1] || st[2]) {
         check(cudaMemsetAsync(fx_state_.get() + 1, 0, 2 * sizeof(int), stream_), "memset");
         synchronize();
@@ -1351,7 +1353,7 @@ FxGuard Engine::fxGuard(int rows, const int* done)
     if (guard_hit_ || (int)guard_flags_.size() != blocks) {  // otherwise no block is marked
         guard_flags_.alloc(blocks);
         check(cudaMemsetAsync(guard_flags_.get(), 0, sizeof(int) * blocks, stream_), "memset");
-        guard_hit_ = false;
+        guard_hit_ = 0;
     }
     FxGuard g{};
     g.lim = fx_lim_.get();

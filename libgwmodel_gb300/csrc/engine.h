@@ -324,7 +324,7 @@ private:
                       bool exclude_self, int wpow, const int* flags, const int* all);
     DevBuf<double> zfx_sum_, fx_lim_;  // fx_lim_: limits of G, then of G2
     DevBuf<int> guard_flags_;
-    bool guard_hit_ = false;             // guard_flags_ marks rows of the last guarded solve
+    int guard_hit_ = 0;                  // guard_flags_ marks rows of the last guarded solve (FxGuard::any)
     bool g_fx_ = false, g2_fx_ = false;  // g_, g2_ hold fixed-point sums
     bool g_flagged_ = false;             // ... whose blocks in fx_flags_ k_contract64 has recomputed
     DevBuf<longlong2> ixy_, pf_ixy_;

@@ -147,7 +147,7 @@ struct FxLimits {
 struct FxGuard {
     const double *lim, *lim2;  // limits of G and, optional, of G2 (fit mode); null: no test
     const int* done;           // optional: 64-row blocks that hold FP64 sums already
-    int *flags, *any;
+    int *flags, *any;          // *any: 1, and 2 for a row that is not one of a single variable of value 0
 };
 
 // The same sums on the tensor cores, in 62-bit fixed point (k_contract_fx.cu):

@@ -9,6 +9,7 @@ import pytest
 import oracle as O
 from libgwmodel_gb300 import Engine
 from parity_util import col_rel, rel
+from test_gpu_mgwr import assert_parity, build
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +92,25 @@ def test_hat_matrix_of_an_indicator(kernel, bw, store, geographic):
         np.testing.assert_allclose(got[3], want[3], rtol=1e-9)
         if store:
             assert np.abs(got[4] - want[4]).max() <= 1e-9 * np.abs(want[4]).max()
+
+
+@pytest.mark.parametrize("elsewhere", [0.0, 0.1])
+@pytest.mark.parametrize("geographic", [False, True])
+def test_multiscale_with_a_sparse_uncentred_column(elsewhere, geographic):
+    """One-variable systems of a column that is 0, or small, away from its region: coefficients, and the traces of
+    the hat matrix that its updates leave."""
+    n = 400
+    x, y, c = problem(n, 6, geographic)
+    rng = np.random.default_rng(8)
+    x = np.asfortranarray(np.column_stack([np.ones(n), np.where(x[:, 2] > 0, 1.0, elsewhere * rng.standard_normal(n))]))
+    y = x @ [1.0, 3.0] + rng.normal(0, 0.3, n)
+    unit = 10.0 if geographic else 1.0
+    bw0 = [30.0 * unit, 7.0 * unit]
+    kw = dict(adaptive=[0, 0], kernel=[O.GAUSSIAN] * 2, centered=[0, 0])
+    # init Specified, approach AIC; the first variable's weight also spans the search of the initial fit
+    ref = O.Problem(x, y, c, geographic=geographic).mgwr(bw0=bw0, init_type=[2, 2], approach=[1, 1], select_threshold=[1e-5] * 2,
+                                                         max_iteration=4, lower=20.0 * unit, upper=60.0 * unit, **kw)
+    alg = build(x, y, c, bw0=bw0, init=[2, 2], approach=[1, 1], geographic=geographic, max_iteration=4,
+                lower=20.0 * unit, upper=60.0 * unit, **kw)
+    alg.fit()
+    assert_parity(alg, ref, capped=4)
