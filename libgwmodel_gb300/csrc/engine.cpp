@@ -531,7 +531,7 @@ void Engine::hatPass(double bw, bool adaptive, int kernel, double* S, int row_ta
     a.bw = bw;
     a.kernel = kernel;
     // v_i = A_i^-1 x_i is large where a column rests on small weights: FP64 ones there too
-    if (fxReady(kernel) && ixy_exact_ && !guard_hit_) {
+    if (fxReady(bw, adaptive, kernel) && ixy_exact_ && !guard_hit_) {
         hat_rows_.alloc(n_);
         a.xy = geographic_ ? nullptr : ixy_.get();
         a.e3 = geographic_ ? ie3_.get() : nullptr;
@@ -588,7 +588,7 @@ bool Engine::hatUpdateFx(double bw, bool adaptive, int kernel, const double* T, 
 {
     // v_i is as large as the variable's weights near i are small, if x_i is not 0 (then the
     // row is 0): weights below 2^-62 would be missing from s_ij = v_i w_ij x_j up to 2^-32
-    if (!fxReady(kernel) || !ixy_exact_ || (guard_hit_ & 2)) return false;
+    if (!fxReady(bw, adaptive, kernel) || !ixy_exact_ || (guard_hit_ & 2)) return false;
     const int tiles = (n_ + kTile - 1) / kTile, groups = (n_ + 63) / 64;
     const size_t bytes = (size_t)tiles * groups * 64 * 256;
     if (!fx_fits(64, tiles)) return false;
@@ -1076,9 +1076,11 @@ bool Engine::withinCap(const std::vector<double>& e) const
 // of the squared distance alone; the other kernels keep the FP64 form, and so do
 // great-circle distances of data wider than a cap of 3,200 km radius, where the
 // polynomials of fx_geo.cuh end.
-bool Engine::fxReady(int kernel)
+bool Engine::fxReady(double bw, bool adaptive, int kernel)
 {
     if (kernel != GW_KERNEL_BISQUARE && kernel != GW_KERNEL_GAUSSIAN) return false;
+    // fixed-point rows need a positive finite threshold (an infinite one weighs every pair 1)
+    if (!adaptive && !(bw > 0.0 && std::isfinite(bw))) return false;
     if (zfx_ready_ && zfx_kind_ == 1 && zfx_bad_ == 1) return false;
     const int tiles = (n_ + kTile - 1) / kTile;
     int groups = 0;
@@ -1381,7 +1383,7 @@ void Engine::contract(const double* Z, int mcols, double* G, int ldg, double bw,
                       bool exclude_self, int wpow, WeightUse use)
 {
     cudaEvent_t e0 = stats_on_ ? timerBegin() : nullptr;
-    const bool fx = fxReady(kernel);
+    const bool fx = fxReady(bw, adaptive, kernel);
     if (use != WeightUse::kAgain) fx_weights_kept_ = false;
     const bool rest = !fx || contractFx(fxFocus(), tb16_.get(), n_, mcols, G, ldg, thrPtr(adaptive), bw, kernel,
                                         exclude_self, wpow, ixy_exact_,
@@ -1864,7 +1866,7 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     }
     // X^T W_i X, X^T W_i y at every location, then beta_i = (X^T W_i X)^-1 X^T W_i y
     pf_g_.alloc((size_t)nr * m_);
-    bool fx = fxReady(kernel), fexact = ixy_exact_;
+    bool fx = fxReady(bw, adaptive, kernel), fexact = ixy_exact_;
     FxLimits limits{};
     if (fx) limits = fxLimits(bw, adaptive, kernel, 1);
     if (fx && geographic_ && withinCap(fe)) {

@@ -292,7 +292,7 @@ private:
     const double* orderStatistic(unsigned rank);
     // Fixed-point contraction of the FP64 form (k_contract_fx.cu): integer
     // coordinates or unit vectors (per dataset), the digit images of Z (per X and y), scratch.
-    bool fxReady(int kernel);
+    bool fxReady(double bw, bool adaptive, int kernel);
     bool integerCoords(int n, const double* u, const double* v, DevBuf<longlong2>& out, bool& exact);
     bool withinCap(const std::vector<double>& e) const;
     bool contractFx(const void* focus, const float4* ftb16, int nf, int mcols, double* G, int ldg, const double* thr,

@@ -267,3 +267,29 @@ def test_geographic_predictions():
     for at in (near, far):
         for kernel in (O.BISQUARE, O.GAUSSIAN):
             assert col_rel(e.predict(at, 90, True, kernel)[:20], ref.predict(at, 90, True, kernel)[:20]) <= 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("geographic", [False, True])
+@pytest.mark.parametrize("kernel", [O.GAUSSIAN, O.BISQUARE])
+def test_infinite_bandwidth(kernel, geographic):
+    """Every pair has weight 1, in the first call on the data and in those after it: criteria, a fit with S and
+    qDiag, predictions, then a finite bandwidth."""
+    x, y, coords = problem(300, 3, 31)
+    g = degrees(coords, 5.0, 45.0, 10.0) if geographic else coords
+    e, ref = engine(x, y, g, geographic), O.Problem(x, y, g, geographic=geographic)
+    inf = float("inf")
+    for bw in (inf, inf, 900.0 if geographic else 120.0, inf):
+        for crit in (O.AIC, O.CV):
+            want, _ = ref.criterion(bw, False, kernel, crit)
+            got = e.criterion(bw, False, kernel, crit)
+            assert abs(got - want) <= 1e-9 * abs(want), (bw, crit, got, want)
+        for store in (True, False):
+            betas, se, shat, qdiag, S = e.fit(bw, False, kernel, store)
+            rb, rse, rshat, rq, rS = ref.fit_core(bw, False, kernel, store)
+            assert col_rel(betas, rb) <= 1e-10
+            assert col_rel(se, rse) <= 1e-9
+            np.testing.assert_allclose(shat, rshat, rtol=1e-9)
+            np.testing.assert_allclose(qdiag, rq, rtol=1e-9)
+            assert np.abs(S - rS).max() <= 1e-9 * np.abs(rS).max()
+        assert col_rel(e.predict(g[:40] + 0.01, bw, False, kernel), ref.predict(g[:40] + 0.01, bw, False, kernel)) <= 1e-10
