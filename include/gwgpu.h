@@ -239,8 +239,8 @@ int gwgpu_engine_set_precision(gwgpu_engine* e, int precision);
 /* Mixed path: 32-point data tiles summed in FP32 on the tensor core before
    each double-float drain (default 64, at least 2). */
 int gwgpu_engine_set_flush_tiles(gwgpu_engine* e, int tiles);
-/* Mixed path: polls of each pipeline wait of the tensor-core contraction before
-   it times out (0 = the default, about two seconds).  A timeout makes the
+/* Polls of each pipeline wait of the tensor-core contractions (mixed, and FP64 in
+   fixed point) before it times out (0 = the default, about two seconds).  A timeout makes the
    kernel wait for its own MMAs and copies, free its tensor memory and report;
    the call then fails with GWGPU_ERR_CUDA and the engine stays usable.  Small
    values are for testing that path (no counterpart in libgwmodel). */

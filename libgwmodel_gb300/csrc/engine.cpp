@@ -1188,6 +1188,7 @@ bool Engine::refineFx(double bw, bool adaptive, int kernel, const float* d2c)
     a.zexp = zfx_exp_.get();
     a.zcols = zfx_n_ * zfx_groups_;
     a.err = fx_state_.get() + 1;
+    a.wait_limit = tc_wait_limit_;
     a.limits = fxLimits(bw, adaptive, kernel, 1);
     // the contraction's sums are free by now: rows of at most npad doubles
     double* G = reinterpret_cast<double*>(acc_.get());
@@ -1233,6 +1234,7 @@ FxArgs Engine::fxArgs(double bw, const double* thr) const
     a.thr = thr;
     a.bw = bw;
     a.err = fx_state_.get() + 1;
+    a.wait_limit = tc_wait_limit_;
     return a;
 }
 

@@ -132,7 +132,7 @@ public:
     void setPrecision(int precision) { precision_ = precision; }
     // Tiles per FP32 accumulation chunk of the tensor-core contraction (>= 2).
     void setFlushTiles(int tiles) { flush_tiles_ = tiles; }
-    // Polls of the tensor-core contraction's pipeline waits before they time out
+    // Polls of the tensor-core contractions' pipeline waits before they time out
     // (0: the default, about two seconds); small values exercise the timeout path.
     void setTcWaitLimit(unsigned polls) { tc_wait_limit_ = polls; }
     int flushTiles() const { return flush_tiles_; }

@@ -181,6 +181,7 @@ struct FxArgs {
     const double* rowscale;     // optional (one split only): row i's sums are multiplied by rowscale[i]
     unsigned* rowmax;           // splits x nf: high words of the largest weight
     int* err;                   // set to 1 if a bounded wait timed out
+    unsigned wait_limit;        // polls of a pipeline wait before it times out (0: the default)
     int group0, groups;         // column groups of this launch (groups 0: all of ncols)
     // Weights kept for further passes over the same rows, points and thresholds: row block x
     // tile x 16 points x 128 rows (fx_weight_bytes); wstore writes them, wload reads them.

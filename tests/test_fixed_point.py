@@ -293,3 +293,25 @@ def test_infinite_bandwidth(kernel, geographic):
             np.testing.assert_allclose(qdiag, rq, rtol=1e-9)
             assert np.abs(S - rS).max() <= 1e-9 * np.abs(rS).max()
         assert col_rel(e.predict(g[:40] + 0.01, bw, False, kernel), ref.predict(g[:40] + 0.01, bw, False, kernel)) <= 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,p,geographic,kernel", [(3000, 9, True, O.GAUSSIAN), (3000, 5, False, O.GAUSSIAN),
+                                                   (2000, 17, False, O.BISQUARE)])
+def test_timeout_is_reported_and_engine_recovers(n, p, geographic, kernel):
+    """With a limit of one poll the contraction's pipeline waits run out: the kernel waits for its own MMAs, commits
+    and bulk copies, frees its tensor memory and sets the error flag; criterion, fit and prediction fail with that
+    error, and the next call on the same engine returns the value it returned before."""
+    from libgwmodel_gb300 import GwgpuError
+    x, y, coords = problem(n, p, n + p)
+    g = degrees(coords, 5.0, 45.0, 20.0) if geographic else coords
+    e = engine(x, y, g, geographic)
+    calls = [lambda: e.criterion(n // 2, True, kernel, O.AIC), lambda: e.criterion(n // 2, True, kernel, O.CV),
+             lambda: e.fit(n // 2, True, kernel, False)[0], lambda: e.predict(g[:300], n // 2, True, kernel)]
+    want = [f() for f in calls]
+    for f, w in zip(calls, want):
+        e.set_tc_wait_limit(1)
+        with pytest.raises(GwgpuError, match="timed out"):
+            f()
+        e.set_tc_wait_limit(0)
+        assert np.array_equal(f(), w)
