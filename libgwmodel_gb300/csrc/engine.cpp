@@ -1681,7 +1681,8 @@ double Engine::golden(bool adaptive, int kernel, int crit, double lower, double 
     return xopt;
 }
 
-size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool adaptive, long long hist_limit)
+size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool adaptive, long long hist_limit,
+                             int num_sms)
 {
     const double N = n, P = p;
     const double m = P * (P + 1) / 2 + P, mm = P * (P + 1) / 2;
@@ -1695,7 +1696,11 @@ size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool ada
     b += 16 * t32 * 32 * (1 + g) + 16 * t32 + 20 * t16;               // point records, tile bounds, tile thresholds
     b += 8 * 256 * m + 8 * 4 * kMaxP * 65;                            // variable-selection scratch
     const double n128 = std::ceil(N / 128) * 128;                    // rows of the contraction's sums
-    if (mixed) b += 8 * N * (P + 1 + m) + t32 * 2 * npad * 128 + 12 * n128 * npad + 4 * N;
+    b += 8 * N * (P + 3) + 28 * N;                                    // the caller's arrays, the ordering's scratch
+    if (mixed) {
+        b += 8 * N * (P + 1 + m) + t32 * 2 * npad * 128 + 4 * N + 12 * std::ceil(N / 256) * (P + 1);
+        b += 12 * n128 * npad;
+    }
     b += 8 * N * (mm + 2 * P + 2) + 8 * N * (2 * P + 1) + 4 * N;      // fit: G2, v, betasSE, qDiag, S row, results
     b += 4 * N;                                                       // deferred rows of the exact select
     {
@@ -1703,9 +1708,11 @@ size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool ada
         // coordinates (a mixed engine holds them too once it predicts)
         int groups = 0;
         const int w = fx_columns((int)m, &groups);
-        const int splits = fx_splits((n + 127) / 128 * groups, (n + 15) / 16, 152);
-        b += 40 * N + 8 * N * hat_splits(n, 152);
-        b += t16 * groups * w * 256 + std::ceil(N / 1024) * groups * w * 4 + 32 * N;
+        int splits = 1;
+        for (int g = 1; g <= groups; g++)
+            splits = std::max(splits, fx_splits((n + 127) / 128 * g, (n + 15) / 16, num_sms));
+        b += 40 * N + 8 * N * hat_splits(n, num_sms);
+        b += t16 * groups * w * 256 + std::ceil(N / 1024) * groups * w * 20 + 32 * N;
         b += (splits > 1 ? 8 * N * m * splits : 0.0) + 4 * N * splits + N;
     }
     if (adaptive) {
@@ -1714,26 +1721,6 @@ size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool ada
         b += 64 * 8 * N;                                              // cached order statistics
     }
     return (size_t)(b * 1.05) + (16u << 20);
-}
-
-size_t Engine::bytesHeld() const
-{
-    size_t b = u_.capacityBytes() + v_.capacityBytes() + uR_.capacityBytes() + vR_.capacityBytes() + e_.capacityBytes() +
-               x_.capacityBytes() + y_.capacityBytes() + z_.capacityBytes() + g_.capacityBytes() +
-               thr_.capacityBytes() + sel0_.capacityBytes() + sel1_.capacityBytes() + beta_.capacityBytes() +
-               sii_.capacityBytes() + resid_.capacityBytes() + partials_.capacityBytes() + fx_weights_.capacityBytes() +
-               tiles_.capacityBytes() + caps_.capacityBytes() + boxes32_.capacityBytes() + caps32_.capacityBytes() +
-               rvec_.capacityBytes() + pts32_.capacityBytes() + tbsel_.capacityBytes() + tb16_.capacityBytes() +
-               tile_thr16_.capacityBytes() + xs_.capacityBytes() + ys_.capacityBytes() + zs_.capacityBytes() +
-               zimg_.capacityBytes() + acc_.capacityBytes() + stage_.capacityBytes() + thr32_.capacityBytes() + g2_.capacityBytes() +
-               vvec_.capacityBytes() + bse_.capacityBytes() + qdiag_.capacityBytes() + S_.capacityBytes() +
-               hist_.capacityBytes() + hcoarse_.capacityBytes() + gall_part_.capacityBytes() + gsub_.capacityBytes() + stb_.capacityBytes() +
-               ixy_.capacityBytes() + ie3_.capacityBytes() + zfx_.capacityBytes() + zfx_exp_.capacityBytes() + fx_flags_.capacityBytes() +
-               fx_part_.capacityBytes() + fx_rowmax_.capacityBytes() + hat_rows_.capacityBytes() + hat_sum_.capacityBytes() +
-               out_.capacityBytes() + d_perm_.capacityBytes() + raw_.capacityBytes() + prep_.capacityBytes() + sel_defer_.capacityBytes();
-    for (auto& r : ranks_) b += r->v.capacityBytes();
-    for (auto& r : rank_pool_) b += r->v.capacityBytes();
-    return b;
 }
 
 void Engine::predict(int nr, const double* locations, double bw, bool adaptive, int kernel,

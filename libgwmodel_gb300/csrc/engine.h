@@ -158,9 +158,9 @@ public:
     // Upper bound of the device memory an engine holds after setData plus a
     // search and a fit of a dataset of this shape (the allocations below), without the
     // buffers of setScratchLimit.
-    static size_t estimateBytes(int n, int p, bool geographic, bool mixed, bool adaptive, long long hist_limit);
-    // Device memory currently held (capacity of every buffer).
-    size_t bytesHeld() const;
+    // num_sms: of the device the engine runs on (the splits of its sums follow from it).
+    static size_t estimateBytes(int n, int p, bool geographic, bool mixed, bool adaptive, long long hist_limit,
+                                int num_sms);
 
     int n() const { return n_; }
     int p() const { return p_; }

@@ -71,12 +71,21 @@ double now_ms(std::chrono::steady_clock::time_point t0)
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// The device's SMs; a GB300's where there is none (an estimate on a host without a GPU).
+int device_sms(int device)
+{
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) return sms;
+    cudaGetLastError();
+    return 152;
+}
+
 }  // namespace
 
 class Server {
 public:
     Server(int device, double budget, int slots)
-        : device_(device), budget_(budget), slots_(slots), reserved_(slots, 0.0), busy_(slots, 0),
+        : device_(device), num_sms_(device_sms(device)), budget_(budget), slots_(slots), reserved_(slots, 0.0), busy_(slots, 0),
           engines_(slots), t0_(std::chrono::steady_clock::now())
     {
         for (int s = 0; s < slots; s++) threads_.emplace_back([this, s] { worker(s); });
@@ -128,7 +137,7 @@ public:
     double estimate(const gwgpu_request& r) const
     {
         return (double)Engine::estimateBytes(r.n, r.p, r.geographic != 0, r.precision == GWGPU_MIXED, r.adaptive != 0,
-                                             hist_limit(r.n));
+                                             hist_limit(r.n), num_sms_);
     }
 
     // 0: done (out filled), 1: timed out, -1: unknown id
@@ -305,7 +314,7 @@ private:
         }
     }
 
-    const int device_;
+    const int device_, num_sms_;
     const double budget_;
     const int slots_;
     std::mutex mu_;
@@ -416,7 +425,8 @@ double gwgpu_server_estimate(gwgpu_server* s, const gwgpu_request* r)
 double gwgpu_estimate_bytes(int n, int p, int geographic, int precision, int adaptive)
 {
     if (n < 1 || p < 1) return 0.0;
-    return (double)gwgpu::Engine::estimateBytes(n, p, geographic != 0, precision == GWGPU_MIXED, adaptive != 0, -1);
+    return (double)gwgpu::Engine::estimateBytes(n, p, geographic != 0, precision == GWGPU_MIXED, adaptive != 0, -1,
+                                                gwgpu::device_sms(0));
 }
 
 int gwgpu_admit_slot(double budget, int slots, const double* reserved, const int* busy, double estimate)

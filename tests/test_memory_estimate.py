@@ -1,0 +1,37 @@
+"""The device memory estimate that admits served requests is an upper bound of what an engine takes for set-up, search
+evaluations and a fit."""
+import numpy as np
+import pytest
+
+import oracle as O
+from libgwmodel_gb300 import Engine, Precision
+from libgwmodel_gb300._lib import lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,p,precision", [(1_500_000, 1, Precision.FP64), (20_011, 17, Precision.FP64),
+                                           (300_000, 2, Precision.Mixed)])
+def test_estimate_covers_a_fit(n, p, precision):
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    x = np.asfortranarray(np.column_stack([np.ones(n), rng.standard_normal((n, p - 1))]))
+    y = x.sum(1) + rng.normal(0, 0.3, n)
+    c = np.asfortranarray(rng.uniform(0, 100, (n, 2)))
+    # a fixed bandwidth that reaches some 60 neighbours and many more at the smallest n
+    bw = 100.0 * np.sqrt((60 + 20 * p) / n)
+    warm = Engine(0)  # the context, the kernels' code and the pinned pages are there before the count
+    warm.set_data(x[:300], y[:300], c[:300], False)
+    warm.set_precision(precision)
+    warm.fit(90.0, False, O.BISQUARE, False)
+    torch.cuda.init()
+    before = torch.cuda.mem_get_info(0)[0]
+    e = Engine(0)
+    e.set_data(x, y, c, False)
+    e.set_precision(precision)
+    kernel = O.BISQUARE if precision == Precision.FP64 else O.GAUSSIAN
+    e.criterion(bw, False, kernel, O.AIC)
+    e.fit(bw, False, kernel, False)
+    held = before - torch.cuda.mem_get_info(0)[0]
+    kept = 4 << 30 if p > 10 else 0  # weights kept for speed, which served engines go without
+    assert held <= lib().gwgpu_estimate_bytes(n, p, 0, int(precision), 0) + kept, (held, p)
