@@ -839,11 +839,18 @@ void Engine::contractMixed(double* G, int ldg, int mcols, double bw, bool adapti
     // the tiles a row block visits: all of them, about twice those that hold the neighbours,
     // or (a fixed bandwidth and a compact kernel) any number: no split
     const bool compact = adaptive && kernel >= GW_KERNEL_BISQUARE;
-    const int visits = compact ? (int)std::min((double)ntiles32_, bw / 16 + 8) : ntiles32_;
+    // (in whole chunks: an estimate of the engine's memory goes through every number)
+    int visits = compact ? (int)std::min((double)ntiles32_, bw / 16 + 8) : ntiles32_;
+    visits = std::min(ntiles32_, (visits + flush_tiles_ - 1) / flush_tiles_ * flush_tiles_);
+    // (the splits group the sums: their number follows from the shape, and from the memory
+    // only where the call would fail for want of it)
     a.nsplit = !adaptive && kernel >= GW_KERNEL_BISQUARE ? 1 : tc_splits((n_ + 127) / 128, visits, flush_tiles_, num_sms_);
-    if (a.nsplit > 1 && !scratchFits(a.nsplit * acc_size * 12, acc_.capacityBytes() + stage_.capacityBytes())) a.nsplit = 1;
-    acc_.alloc(a.nsplit * acc_size);
-    stage_.alloc(a.nsplit * acc_size);
+    if (!acc_.tryAlloc(a.nsplit * acc_size) || !stage_.tryAlloc(a.nsplit * acc_size)) {
+        a.nsplit = 1;
+        acc_.release();
+        acc_.alloc(acc_size);
+        stage_.alloc(acc_size);
+    }
     a.acc_stride = acc_size;
     a.acc = acc_.get();
     a.stage = stage_.get();
@@ -1293,7 +1300,8 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
         if (store) fx_weights_.alloc(bytes / sizeof(unsigned long long));
         fx_weights_kept_ = store && use == WeightUse::kKept;
     }
-    const int nsplit = fx_splits((nf + 127) / 128 * (store ? 1 : groups), a.ntiles, num_sms_);
+    // (the splits group the sums: the same number whether or not the weights fit)
+    const int nsplit = fx_splits((nf + 127) / 128 * (use == WeightUse::kAgain ? groups : 1), a.ntiles, num_sms_);
     fx_rowmax_.alloc((size_t)nsplit * nf);
     a.rowmax = fx_rowmax_.get();
     if (nsplit > 1) {
@@ -1699,7 +1707,11 @@ size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool ada
     b += 8 * N * (P + 3) + 28 * N;                                    // the caller's arrays, the ordering's scratch
     if (mixed) {
         b += 8 * N * (P + 1 + m) + t32 * 2 * npad * 128 + 4 * N + 12 * std::ceil(N / 256) * (P + 1);
-        b += 12 * n128 * npad;
+        // sums and their splits at any number of visited tiles, 64 tiles a chunk
+        int splits = 1;
+        for (int visits = 64; visits < (int)t32 + 64; visits += 64)
+            splits = std::max(splits, tc_splits((int)(n128 / 128), std::min(visits, (int)t32), 64, num_sms));
+        b += 12 * n128 * npad * splits;
     }
     b += 8 * N * (mm + 2 * P + 2) + 8 * N * (2 * P + 1) + 4 * N;      // fit: G2, v, betasSE, qDiag, S row, results
     b += 4 * N;                                                       // deferred rows of the exact select
@@ -1708,7 +1720,7 @@ size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool ada
         // coordinates (a mixed engine holds them too once it predicts)
         int groups = 0;
         const int w = fx_columns((int)m, &groups);
-        int splits = 1;
+        int splits = 1;  // of a first pass (one group's rows) and of passes that read kept weights
         for (int g = 1; g <= groups; g++)
             splits = std::max(splits, fx_splits((n + 127) / 128 * g, (n + 15) / 16, num_sms));
         b += 40 * N + 8 * N * hat_splits(n, num_sms);

@@ -56,6 +56,22 @@ public:
         if (count) check(cudaMalloc(&ptr_, count * sizeof(T)), "cudaMalloc");
         count_ = cap_ = count;
     }
+    // alloc, or false (and empty) when the device has no room.
+    bool tryAlloc(size_t count)
+    {
+        if (count <= cap_ && ptr_) {
+            count_ = count;
+            return true;
+        }
+        release();
+        if (count && cudaMalloc(&ptr_, count * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError();
+            ptr_ = nullptr;
+            return false;
+        }
+        count_ = cap_ = count;
+        return true;
+    }
     // Empty (get() returns null) without freeing the allocation.
     void clear() { count_ = 0; }
     void release()
@@ -147,8 +163,8 @@ public:
     // lets it take up to a quarter of the free device memory.
     void setHistLimit(long long bytes) { hist_limit_bytes_ = bytes; }
     // Largest buffer (bytes) held for speed alone (fixed-point weights that a later pass of
-    // the same call reads back, the splits of a mixed contraction); 0: none.  Never more
-    // than an eighth of the free device memory.
+    // the same call reads back: no sum depends on it); 0: none.  Never more than an eighth of
+    // the free device memory.
     void setScratchLimit(long long bytes) { scratch_limit_bytes_ = bytes; }
     void releaseScratch()
     {

@@ -275,7 +275,7 @@ private:
             if (!engines_[slot]) engines_[slot].reset(new Engine(device_));
             Engine& e = *engines_[slot];
             e.setHistLimit(hist_limit(r.n));
-            e.setScratchLimit(0);        // as the next:
+            e.setScratchLimit(0);        // as the next (results do not depend on it):
             e.setDistanceCacheLimit(0);  // n^2 bytes per request would break the HBM budget's admission
             e.setData(r.n, r.p, q.x.data(), q.y.data(), q.coords.data(), r.geographic != 0);
             e.setPrecision(r.precision == GWGPU_MIXED ? kMixed : kFP64);

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,p,precision", [(1_500_000, 1, Precision.FP64), (20_011, 17, Precision.FP64),
-                                           (300_000, 2, Precision.Mixed)])
+                                           (300_000, 2, Precision.Mixed), (30_011, 9, Precision.Mixed)])
 def test_estimate_covers_a_fit(n, p, precision):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(n)
