@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <mutex>
 #include <numeric>
@@ -269,16 +270,54 @@ void free_d2c(DeviceD2Cache& c)
     c.owner = nullptr;
 }
 
+// The kept weights of each device (Engine::takeWeights), with the engines alive on it.
+struct DeviceWeights {
+    std::mutex mu;
+    std::condition_variable idle;
+    unsigned long long* ptr = nullptr;
+    size_t bytes = 0;
+    const Engine* user = nullptr;  // between the passes of a call
+    cudaEvent_t used = nullptr;    // the last user's last launch
+    int engines = 0;
+};
+DeviceWeights* const g_weights = new DeviceWeights[kMaxDevices];
+
+// (the caller holds the lock, and nobody uses the buffer)
+void free_weights(DeviceWeights& w)
+{
+    if (w.ptr) {
+        cudaEventSynchronize(w.used);
+        cudaFree(w.ptr);
+    }
+    w.ptr = nullptr;
+    w.bytes = 0;
+}
+
 }  // namespace
+
+bool release_idle_scratch()
+{
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return false;
+    DeviceWeights& w = g_weights[device];
+    std::lock_guard<std::mutex> lk(w.mu);
+    if (w.user || !w.ptr) return false;
+    free_weights(w);
+    return true;
+}
 
 Engine::Engine(int device) : device_(device)
 {
     check(cudaSetDevice(device), "cudaSetDevice");
+    if (device >= kMaxDevices) throw std::invalid_argument("device ordinal out of range");
     cudaDeviceProp prop;
     check(cudaGetDeviceProperties(&prop, device), "cudaGetDeviceProperties");
     num_sms_ = prop.multiProcessorCount;
     check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     check(cudaMallocHost(&host_sums_, 8 * sizeof(double)), "cudaMallocHost");
+    DeviceWeights& w = g_weights[device_];
+    std::lock_guard<std::mutex> lk(w.mu);
+    w.engines++;
 }
 
 Engine::~Engine()
@@ -290,6 +329,15 @@ Engine::~Engine()
         if (c.owner == this) {
             cudaSetDevice(device_);
             free_d2c(c);
+        }
+    }
+    {
+        leaveWeights();
+        DeviceWeights& w = g_weights[device_];
+        std::lock_guard<std::mutex> lk(w.mu);
+        if (--w.engines == 0) {
+            cudaSetDevice(device_);
+            free_weights(w);
         }
     }
     for (auto& e : events_)
@@ -506,10 +554,12 @@ void Engine::fitDevice(double bw, bool adaptive, int kernel, bool se, double* ai
     bse_.alloc((size_t)n * p);
     qdiag_.alloc(n);
     computeThresholds(bw, adaptive);
-    contract(z_.get(), m_, g_.get(), m_, bw, adaptive, kernel, false, 1, se ? WeightUse::kKept : WeightUse::kOnce);
-    if (se)
-        contract(z_.get(), mm_, g2_.get(), mm_, bw, adaptive, kernel, false, 2, WeightUse::kAgain);
-    else  // the solve still forms the (unused) SE terms from G2
+    {
+        WeightScope scope{*this};
+        contract(z_.get(), m_, g_.get(), m_, bw, adaptive, kernel, false, 1, se ? WeightUse::kKept : WeightUse::kOnce);
+        if (se) contract(z_.get(), mm_, g2_.get(), mm_, bw, adaptive, kernel, false, 2, WeightUse::kAgain);
+    }
+    if (!se)  // the solve still forms the (unused) SE terms from G2
         check(cudaMemsetAsync(g2_.get(), 0, sizeof(double) * g2_.size(), stream_), "memset G2");
     ainv_out_ = ainv;
     double s[4];
@@ -595,7 +645,9 @@ bool Engine::hatUpdateFx(double bw, bool adaptive, int kernel, const double* T, 
     if (hat_img_.capacityBytes() < bytes) {
         size_t free_b = 0, total_b = 0;
         check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-        if (bytes + (bytes >> 3) + (1u << 30) > free_b) return false;
+        const auto fits = [&] { return bytes + (bytes >> 3) + (1u << 30) <= free_b; };
+        if (!fits() && release_idle_scratch()) check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+        if (!fits()) return false;
         hat_img_.alloc(bytes);
     }
     hat_exp_.alloc((size_t)((n_ + 1023) / 1024) * groups * 64);
@@ -934,6 +986,10 @@ const double* Engine::orderStatistic(unsigned rank)
             size_t free_b = 0, total_b = 0;
             cudaMemGetInfo(&free_b, &total_b);
             fits = bytes < free_b / 4 || bytes <= hist_.capacityBytes() + hcoarse_.capacityBytes();
+            if (!fits && release_idle_scratch()) {
+                cudaMemGetInfo(&free_b, &total_b);
+                fits = bytes < free_b / 4;
+            }
         }
         if (fits) {
             hist_.alloc((size_t)n_ * 4096);
@@ -1255,6 +1311,43 @@ void Engine::setFocus(FxArgs& a, const void* focus, const float4* ftb16, int nf,
     a.exact = exact ? 1 : 0;
 }
 
+// The device's buffer for kept weights (bytes), or null where it may not grow to that size.
+// Waits for an engine that is between its passes: on the host for the launches of the
+// other passes, on the stream for their end.
+unsigned long long* Engine::takeWeights(size_t bytes)
+{
+    if (bytes > (size_t)scratch_limit_bytes_) return nullptr;
+    DeviceWeights& w = g_weights[device_];
+    std::unique_lock<std::mutex> lk(w.mu);
+    w.idle.wait(lk, [&] { return !w.user || w.user == this; });
+    if (w.bytes < bytes) {
+        free_weights(w);
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes >= free_b / 8 ||
+            cudaMalloc(&w.ptr, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            w.ptr = nullptr;
+            return nullptr;
+        }
+        w.bytes = bytes;
+    }
+    if (!w.used) check(cudaEventCreateWithFlags(&w.used, cudaEventDisableTiming), "cudaEventCreate");
+    check(cudaStreamWaitEvent(stream_, w.used, 0), "cudaStreamWaitEvent");
+    w.user = this;
+    return w.ptr;
+}
+
+void Engine::leaveWeights()
+{
+    DeviceWeights& w = g_weights[device_];
+    std::lock_guard<std::mutex> lk(w.mu);
+    fx_weights_kept_ = false;
+    if (w.user != this) return;
+    cudaEventRecord(w.used, stream_);
+    w.user = nullptr;
+    w.idle.notify_all();
+}
+
 // G over the first mcols columns of Z by the fixed-point contraction, for the
 // focus rows given as integer coordinates and tile bounds.  Returns whether
 // fx_flags_ now marks row blocks for k_contract64: rows that exclude their own
@@ -1262,16 +1355,6 @@ void Engine::setFocus(FxArgs& a, const void* focus, const float4* ftb16, int nf,
 // coordinates may be too coarse for a small threshold; every other row holds its
 // own weight 1.  Until the first synchronisation has told whether Z suits, the
 // FP64 kernel is launched behind it too (it leaves at once when it does).
-// Whether a buffer held for speed alone may grow from `held` bytes to `bytes`.
-bool Engine::scratchFits(size_t bytes, size_t held) const
-{
-    if (bytes > (size_t)scratch_limit_bytes_) return false;
-    if (bytes <= held) return true;
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    return bytes < free_b / 8;
-}
-
 bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcols, double* G, int ldg,
                         const double* thr, double bw, int kernel, bool exclude_self, int wpow, bool exact,
                         const FxLimits& limits, WeightUse use)
@@ -1292,14 +1375,10 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
     // Further column groups and passes read the first group's weights back: making them
     // takes some 10 times as long as the rest of a tile (n = 20,011, p = 17, great-circle).
     const bool load = use == WeightUse::kAgain && fx_weights_kept_;
-    if (load) fx_weights_kept_ = false;
-    bool store = false;
-    if (!load && (groups > 1 || use == WeightUse::kKept)) {
-        const size_t bytes = fx_weight_bytes(nf, n_);
-        store = scratchFits(bytes, fx_weights_.capacityBytes());
-        if (store) fx_weights_.alloc(bytes / sizeof(unsigned long long));
-        fx_weights_kept_ = store && use == WeightUse::kKept;
-    }
+    const bool wanted = load || groups > 1 || use == WeightUse::kKept;
+    unsigned long long* const weights = wanted ? takeWeights(fx_weight_bytes(nf, n_)) : nullptr;
+    const bool store = weights && !load;
+    if (use == WeightUse::kKept) fx_weights_kept_ = store;
     // (the splits group the sums: the same number whether or not the weights fit)
     const int nsplit = fx_splits((nf + 127) / 128 * (use == WeightUse::kAgain ? groups : 1), a.ntiles, num_sms_);
     fx_rowmax_.alloc((size_t)nsplit * nf);
@@ -1314,9 +1393,9 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
         a.ldo = ldg;
     }
     if (flags) fx_flags_.alloc((nf + kRowBlock - 1) / kRowBlock);
-    if (load) a.wload = fx_weights_.get();
+    if (load) a.wload = weights;
     if (store) {
-        a.wstore = fx_weights_.get();
+        a.wstore = weights;
         a.groups = 1;
     }
     check(launch_contract_fx(a, fxMode(kernel), nsplit, stream_), "contract_fx");
@@ -1328,6 +1407,7 @@ bool Engine::contractFx(const void* focus, const float4* ftb16, int nf, int mcol
         check(launch_contract_fx(a, fxMode(kernel), nsplit, stream_), "contract_fx");
         stats_.kernel_launches += 1;
     }
+    if (weights && !fx_weights_kept_) leaveWeights();
     check(launch_fx_finish(a, nsplit, G, ldg, flags ? fx_flags_.get() : nullptr, stream_), "fx_finish");
     stats_.kernel_launches += nsplit > 1 || flags ? 2 : 1;
     return flags;
@@ -1394,7 +1474,6 @@ void Engine::contract(const double* Z, int mcols, double* G, int ldg, double bw,
 {
     cudaEvent_t e0 = stats_on_ ? timerBegin() : nullptr;
     const bool fx = fxReady(bw, adaptive, kernel);
-    if (use != WeightUse::kAgain) fx_weights_kept_ = false;
     const bool rest = !fx || contractFx(fxFocus(), tb16_.get(), n_, mcols, G, ldg, thrPtr(adaptive), bw, kernel,
                                         exclude_self, wpow, ixy_exact_,
                                         fxLimits(bw, adaptive, kernel, wpow), use);
@@ -1584,6 +1663,7 @@ void Engine::fit(double bw, bool adaptive, int kernel, bool storeS, FitOutput& o
         contractMixed(g_.get(), m_, m_, bw, adaptive, kernel, false, 1);
         contractMixed(g2_.get(), mm_, mm_, bw, adaptive, kernel, false, 2);
     } else {
+        WeightScope scope{*this};
         contract(z_.get(), m_, g_.get(), m_, bw, adaptive, kernel, false, 1, WeightUse::kKept);
         contract(z_.get(), mm_, g2_.get(), mm_, bw, adaptive, kernel, false, 2, WeightUse::kAgain);
     }
@@ -1994,6 +2074,7 @@ float* Engine::acquireDistanceCache()
             return nullptr;
         }
         const size_t reserve = std::max((size_t)16 << 30, total_b / 8);
+        if (need + reserve > free_b && release_idle_scratch()) cudaMemGetInfo(&free_b, &total_b);
         if (need + reserve > free_b) return nullptr;
         if (cudaMalloc(&c.ptr, need) != cudaSuccess) {
             cudaGetLastError();  // too little memory after all: run without the cache

@@ -36,6 +36,10 @@ struct NotSPDError : std::runtime_error {
 
 void check(cudaError_t e, const char* what);
 
+// Gives back what the current device holds for speed alone and nobody is using (the kept
+// weights of setScratchLimit); whether there was anything.
+bool release_idle_scratch();
+
 template <class T>
 class DevBuf {
 public:
@@ -53,7 +57,12 @@ public:
             return;
         }
         release();
-        if (count) check(cudaMalloc(&ptr_, count * sizeof(T)), "cudaMalloc");
+        cudaError_t rc = count ? cudaMalloc(&ptr_, count * sizeof(T)) : cudaSuccess;
+        if (rc == cudaErrorMemoryAllocation && release_idle_scratch()) {
+            cudaGetLastError();
+            rc = cudaMalloc(&ptr_, count * sizeof(T));
+        }
+        check(rc, "cudaMalloc");
         count_ = cap_ = count;
     }
     // alloc, or false (and empty) when the device has no room.
@@ -164,13 +173,9 @@ public:
     void setHistLimit(long long bytes) { hist_limit_bytes_ = bytes; }
     // Largest buffer (bytes) held for speed alone (fixed-point weights that a later pass of
     // the same call reads back: no sum depends on it); 0: none.  Never more than an eighth of
-    // the free device memory.
+    // the free device memory.  One buffer per device serves its engines in turn; it is given
+    // back with the last of them, and when an allocation needs the room.
     void setScratchLimit(long long bytes) { scratch_limit_bytes_ = bytes; }
-    void releaseScratch()
-    {
-        fx_weights_.release();
-        fx_weights_kept_ = false;
-    }
     // Upper bound of the device memory an engine holds after setData plus a
     // search and a fit of a dataset of this shape (the allocations below), without the
     // buffers of setScratchLimit.
@@ -298,9 +303,14 @@ private:
         ranks_.clear();
     }
     long long scratch_limit_bytes_ = 4ll << 30;
-    DevBuf<unsigned long long> fx_weights_;
     bool fx_weights_kept_ = false;
-    bool scratchFits(size_t bytes, size_t held) const;
+    unsigned long long* takeWeights(size_t bytes);
+    void leaveWeights();
+    // The device's buffer is this engine's until the end of the scope at the latest.
+    struct WeightScope {
+        Engine& e;
+        ~WeightScope() { e.leaveWeights(); }
+    };
     long long hist_limit_bytes_ = -1;  // histogram cache limit; -1: a quarter of the free memory
     DevBuf<unsigned> hist_;    // per-row histograms of proxy distances (n x 4096)
     DevBuf<unsigned> hcoarse_; // their cumulative counts per 64-bin segment (n x 64)

@@ -280,8 +280,8 @@ mat GWRMultiscale::fit()
         gwgpu::check(cudaMemGetInfo(&freeb, &total), "cudaMemGetInfo");
         const double held = (double)(I.S0.capacityBytes() + I.SA.capacityBytes() + I.T.capacityBytes() +
                                      I.ainv.capacityBytes());
-        if (need > (double)freeb + held) {  // what the engine holds for speed alone goes first
-            eng.releaseScratch();
+        if (need > (double)freeb + held) {  // what is held for speed alone goes first
+            gwgpu::release_idle_scratch();
             gwgpu::check(cudaMemGetInfo(&freeb, &total), "cudaMemGetInfo");
         }
         if (need > (double)freeb + held)
