@@ -43,4 +43,11 @@ uint64_t fx_ratio63(uint64_t num, uint64_t den) { return ratio63(num, den); }
 
 uint64_t fx_square(uint64_t w) { return square(w); }
 
+double fx_squares(const float* s, int n, double acc)
+{
+    Squares q;
+    for (int i = 0; i < n; i++) q.add(s[i]);
+    return q.any() ? q.add_to(acc) : acc;
+}
+
 }
