@@ -177,7 +177,7 @@ public:
     Status status() const { return mStatus; }
     bool isValid();
 
-    mat fit() { return fitInPlace(); }
+    mat fit();
     // fit() without a copy of the coefficients: betas(), or zeros when stopped.
     const mat& fitInPlace();
     // GWRBasic::predict (GWRBasic.cpp:130-155): coefficients at the given
@@ -200,7 +200,7 @@ private:
     double bandwidthCriterion(const BandwidthWeight& w);
     double indepVarsCriterion(const std::vector<std::size_t>& vars, const std::function<double()>& criterion);
 
-    mat mX, mCoords, mBetas, mBetasSE, mS, mStopped;
+    mat mX, mCoords, mBetas, mBetasSE, mS;
     vec mY, mSHat, mQDiag;
     SpatialWeight mSpatialWeight;
     bool mHasIntercept = true, mHasHatMatrix = true;

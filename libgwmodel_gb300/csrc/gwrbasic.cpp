@@ -23,6 +23,7 @@ const char* kFile = "gwrbasic.cpp";
 struct GWRBasic::Impl {
     std::unique_ptr<gwgpu::Engine> engine;
     int device = -1;
+    mat stopped;  // what fitInPlace() returns when the telegram stops it
 };
 
 #define GW_LOG(LEVEL, MSG) mTelegram->print((MSG), ITelegram::LogLevel::LEVEL, __func__, kFile)
@@ -132,6 +133,8 @@ double GWRBasic::indepVarsCriterion(const std::vector<std::size_t>& vars, const 
     return DBL_MAX;
 }
 
+mat GWRBasic::fit() { return fitInPlace(); }
+
 const mat& GWRBasic::fitInPlace()
 {
     GW_STAGE("Initializing");
@@ -147,7 +150,7 @@ const mat& GWRBasic::fitInPlace()
     gwgpu::Engine& eng = *mImpl->engine;
     eng.setPrecision((int)mPrecision);
     eng.setData((int)nDp, (int)nVars, mX.memptr(), mY.memptr(), mCoords.memptr(), geographic);
-    GW_STOP_RETURN(mStopped = mat(nDp, nVars));
+    GW_STOP_RETURN(mImpl->stopped = mat(nDp, nVars));
 
     if (mIsAutoselectIndepVars) {
         GW_STAGE("Independent variable selection");
@@ -223,7 +226,7 @@ const mat& GWRBasic::fitInPlace()
                 eng.setVariables((int)nVars, mX.memptr(), mY.memptr());  // the same points
             }
         }
-        GW_STOP_RETURN(mStopped = mat(nDp, nVars));
+        GW_STOP_RETURN(mImpl->stopped = mat(nDp, nVars));
     }
 
     if (mIsAutoselectBandwidth) {
@@ -252,13 +255,13 @@ const mat& GWRBasic::fitInPlace()
             mSpatialWeight.setWeight(wopt);
             mBandwidthSelectionCriterionList.assign(record.begin(), record.end());
         }
-        GW_STOP_RETURN(mStopped = mat(nDp, nVars));
+        GW_STOP_RETURN(mImpl->stopped = mat(nDp, nVars));
     }
 
     GW_STAGE("Model fitting");
     const BandwidthWeight& bw = *mSpatialWeight.weight();
     const bool storeS = mHasHatMatrix && nDp < 8192;  // isStoreS (GWRBasic.h:708)
-    GW_STOP_RETURN(mStopped = mat(nDp, nVars));
+    GW_STOP_RETURN(mImpl->stopped = mat(nDp, nVars));
     gwgpu::FitOutput out;
     try {
         eng.fit(bw.bandwidth(), bw.adaptive(), (int)bw.kernel(), storeS, out);
@@ -272,7 +275,7 @@ const mat& GWRBasic::fitInPlace()
     mSHat = vec(2, 1, out.shat);
     mQDiag = vec(nDp, 1, std::move(out.qdiag));
     mS = mat((std::size_t)out.sRows, nDp, std::move(out.S));
-    GW_STOP_RETURN(mStopped = mat(nDp, nVars));
+    GW_STOP_RETURN(mImpl->stopped = mat(nDp, nVars));
 
     GW_STAGE("Model Diagnostic");
     // CalcDiagnostic (GWRBasic.cpp:21-34)
