@@ -164,71 +164,33 @@ void split_fp32(double v, float& hi, float& lo)
     lo = (float)(v - (double)hi);
 }
 
-// FP32 records of the points (hu, hv), padded to whole 32-point tiles: planar
-// (u - uc, v - vc) split hi/lo in one float4; geographic the unit vector split
-// hi/lo in two float4 (its z is sin(lat)).
-// e: the points' unit vectors (3 x n), geographic only.
-std::vector<float4> point_records(const std::vector<double>& hu, const std::vector<double>& hv, bool geographic,
-                                  double uc, double vc, const std::vector<double>& e)
+// FP32 records of geographic points, padded to whole 32-point tiles: the unit vector (e:
+// 3 x n) split hi/lo in two float4 (its z is sin(lat)).  Planar ones: k_planar_proxy.
+std::vector<float4> point_records(const std::vector<double>& e)
 {
-    const int n = (int)hu.size();
-    const size_t nt32 = (size_t)(n + 31) / 32;
-    std::vector<float4> pts;
-    if (!geographic) {
-        pts.assign(nt32 * 32, make_float4(0.f, 0.f, 0.f, 0.f));
-        parallel_for((size_t)n, 8192, [&](size_t b, size_t en) {
-            for (size_t s = b; s < en; s++) {
-                float a, bb, c, d;
-                split_fp32(hu[s] - uc, a, bb);
-                split_fp32(hv[s] - vc, c, d);
-                pts[s] = make_float4(a, bb, c, d);
-            }
-        });
-    } else {
-        pts.assign(2 * nt32 * 32, make_float4(0.f, 0.f, 0.f, 0.f));
-        parallel_for((size_t)n, 8192, [&](size_t b, size_t en) {
-            for (size_t s = b; s < en; s++) {
-                float xh, xl, yh, yl, zh, zl;
-                split_fp32(e[s], xh, xl);
-                split_fp32(e[(size_t)n + s], yh, yl);
-                split_fp32(e[2 * (size_t)n + s], zh, zl);
-                pts[2 * s] = make_float4(xh, yh, zh, 0.f);
-                pts[2 * s + 1] = make_float4(xl, yl, zl, 0.f);
-            }
-        });
-    }
+    const size_t n = e.size() / 3, nt32 = (n + 31) / 32;
+    std::vector<float4> pts(2 * nt32 * 32, make_float4(0.f, 0.f, 0.f, 0.f));
+    parallel_for(n, 8192, [&](size_t b, size_t en) {
+        for (size_t s = b; s < en; s++) {
+            float xh, xl, yh, yl, zh, zl;
+            split_fp32(e[s], xh, xl);
+            split_fp32(e[n + s], yh, yl);
+            split_fp32(e[2 * n + s], zh, zl);
+            pts[2 * s] = make_float4(xh, yh, zh, 0.f);
+            pts[2 * s + 1] = make_float4(xl, yl, zl, 0.f);
+        }
+    });
     return pts;
 }
 
-// FP32 bounds of consecutive tiles of `size` points, rounded outward: planar
-// boxes relative to (uc, vc) widened by `slack`, geographic 3-D caps.
-
-std::vector<float4> tile_bounds(const std::vector<double>& hu, const std::vector<double>& hv, bool geographic,
-                                int size, double uc, double vc, double slack, const std::vector<double>& e)
+// FP32 caps of consecutive tiles of `size` geographic points, rounded outward.
+std::vector<float4> tile_bounds(const std::vector<double>& e, int size)
 {
-    const int n = (int)hu.size();
-    const int nt = (n + size - 1) / size;
-    std::vector<float4> tb(nt);
-    if (!geographic) {
-        for (int t = 0; t < nt; t++) {
-            double ulo = hu[t * size], uhi = ulo, vlo = hv[t * size], vhi = vlo;
-            for (int s = t * size; s < std::min(n, (t + 1) * size); s++) {
-                ulo = std::min(ulo, hu[s]);
-                uhi = std::max(uhi, hu[s]);
-                vlo = std::min(vlo, hv[s]);
-                vhi = std::max(vhi, hv[s]);
-            }
-            tb[t] = make_float4(nextafterf((float)(ulo - uc - slack), -INFINITY),
-                                nextafterf((float)(uhi - uc + slack), INFINITY),
-                                nextafterf((float)(vlo - vc - slack), -INFINITY),
-                                nextafterf((float)(vhi - vc + slack), INFINITY));
-        }
-    } else {
-        std::vector<TileCap> cp = make_caps(e, size);
-        for (int t = 0; t < nt; t++)
-            tb[t] = make_float4((float)cp[t].cx, (float)cp[t].cy, (float)cp[t].cz,
-                                nextafterf((float)cp[t].rho, INFINITY) * (1.0f + 1e-6f) + 1e-7f);
-    }
+    const std::vector<TileCap> cp = make_caps(e, size);
+    std::vector<float4> tb(cp.size());
+    for (size_t t = 0; t < cp.size(); t++)
+        tb[t] = make_float4((float)cp[t].cx, (float)cp[t].cy, (float)cp[t].cz,
+                            nextafterf((float)cp[t].rho, INFINITY) * (1.0f + 1e-6f) + 1e-7f);
     return tb;
 }
 
@@ -740,12 +702,12 @@ void Engine::buildProxy()
               "planar records and bounds");
         stats_.kernel_launches += 1;
     } else {
-        const std::vector<float4> pts = point_records(hu_, hv_, true, 0.0, 0.0, he_);
+        const std::vector<float4> pts = point_records(he_);
         const std::vector<TileCap> c32 = make_caps(he_, 32);
         const std::vector<TileBox> bx = make_boxes(hu_, hv_, 32);
-        const std::vector<float4> tb = tile_bounds(hu_, hv_, true, 32, 0.0, 0.0, 0.0, he_);
-        const std::vector<float4> t16 = tile_bounds(hu_, hv_, true, kTile, 0.0, 0.0, 0.0, he_);
-        const std::vector<float4> t1024 = tile_bounds(hu_, hv_, true, 1024, 0.0, 0.0, 0.0, he_);
+        const std::vector<float4> tb = tile_bounds(he_, 32);
+        const std::vector<float4> t16 = tile_bounds(he_, kTile);
+        const std::vector<float4> t1024 = tile_bounds(he_, 1024);
         caps32_.alloc(c32.size());
         auto up = [&](void* dst, const void* src, size_t bytes) {
             check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_), "H2D tile bounds");
@@ -1124,14 +1086,12 @@ bool Engine::integerCoords(int n, const double* u, const double* v, DevBuf<longl
 bool Engine::withinCap(const std::vector<double>& e) const
 {
     const size_t n = e.size() / 3;
-    double far = 0.0;
     for (size_t i = 0; i < n; i++) {
         const double dx = e[i] - ec_[0], dy = e[n + i] - ec_[1], dz = e[2 * n + i] - ec_[2];
         const double d = dx * dx + dy * dy + dz * dz;
         if (!(d < 0.2499)) return false;
-        far = std::max(far, d);
     }
-    return far < 0.2499;
+    return true;
 }
 
 // Whether the fixed-point contraction applies to the resident data and kernel;
@@ -1585,7 +1545,8 @@ void Engine::solve(int mode, double bw, bool adaptive, int kernel, double out[4]
 }
 
 // One refinement step of every local solve (mixed path): residual of the
-// normal equations in FP64 over the contraction's weights, then beta += A~^-1 r.
+// normal equations over the contraction's FP32 weights (exact sums, or the double-float
+// pass where those do not apply), then beta += A~^-1 r.
 void Engine::refine(double bw, bool adaptive, int kernel, double out[4])
 {
     RefineArgs r{};
@@ -1863,18 +1824,16 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
               "planar records and bounds");
         stats_.kernel_launches += 1;
     } else {
-        std::vector<double> fu(nr), fv(nr), fuR(nr), fvR(nr);
+        std::vector<double> fuR(nr), fvR(nr);
         auto down = [&](std::vector<double>& dst, const double* src) {
             check(cudaMemcpyAsync(dst.data(), src, sizeof(double) * nr, cudaMemcpyDeviceToHost, stream_), "D2H");
         };
-        down(fu, pf_u_.get());
-        down(fv, pf_v_.get());
         down(fuR, pf_uR_.get());
         down(fvR, pf_vR_.get());
         synchronize();
         fe = unit_vectors(fuR, fvR);
-        const std::vector<float4> fpts = point_records(fu, fv, true, 0.0, 0.0, fe);
-        const std::vector<float4> ftb = tile_bounds(fu, fv, true, kTile, 0.0, 0.0, 0.0, fe);
+        const std::vector<float4> fpts = point_records(fe);
+        const std::vector<float4> ftb = tile_bounds(fe, kTile);
         pf_e_.alloc(fe.size());
         check(cudaMemcpyAsync(pf_e_.get(), fe.data(), sizeof(double) * fe.size(), cudaMemcpyHostToDevice, stream_),
               "H2D unit vectors");

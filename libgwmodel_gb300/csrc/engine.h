@@ -147,7 +147,7 @@ public:
     // SA_k and S0 of the initial all-variable fit from fitDevice's inverses.
     void hatAll(double bw, bool adaptive, int kernel, const double* ainv, double* S0, double* SA);
     // SA = S (T + I) with S the hat matrix of the last one-variable fitDevice
-    // at this bandwidth (a compact kernel), over neighbouring tiles only.
+    // at this bandwidth, over the tiles that hold weight.
     void hatUpdate(double bw, bool adaptive, int kernel, const double* T, double* SA);
     void synchronizeFx();      // synchronize(), and throws if a fixed-point contraction timed out
     void releaseHatScratch();  // hatUpdate's digit images

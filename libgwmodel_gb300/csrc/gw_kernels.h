@@ -460,9 +460,9 @@ cudaError_t launch_mgwr_hat_all(const DevPoints& P, bool geographic, const doubl
                                 cudaStream_t stream);
 // T = SA - S0 over count elements.
 cudaError_t launch_mgwr_sub(size_t count, const double* SA, const double* S0, double* T, cudaStream_t stream);
-// SA = S (T + I) for the one-variable hat matrix S(i, j) = w_ij v_i x_j of a
-// compact kernel (bisquare, tricube, boxcar), over neighbouring data tiles only
-// (X: the variable, v: A_i^-1 x_i from the fit, both n sorted).  With unless, only
+// SA = S (T + I) for the one-variable hat matrix S(i, j) = w_ij v_i x_j, over
+// neighbouring data tiles only where the kernel is compact (bisquare, tricube,
+// boxcar) (X: the variable, v: A_i^-1 x_i from the fit, both n sorted).  With unless, only
 // when *unless is nonzero.
 cudaError_t launch_mgwr_hat_update(const DevPoints& P, bool geographic, const float4* tb16, const double* X,
                                    const double* v, const double* thr, double bw, int kernel, const double* T,

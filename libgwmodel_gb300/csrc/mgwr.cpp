@@ -437,9 +437,8 @@ mat GWRMultiscale::fit()
         I.releaseHat();  // (p + 2) n^2 doubles: not held past the fit
     }
     mDiagnostic = CalcDiagnostic(x, mY, trS, trStS, mRSS0);
-    // this library's kernels (the DGEMMs are cuBLAS's): the engine's (including
-    // the sparse hat updates), plus the two elementwise passes of each hat
-    // update and the final trace reduction
+    // the kernels launched: the engine's (including the hat updates), plus the two
+    // elementwise passes of each hat update and the final trace reduction
     mCounters.kernelLaunches =
         eng.stats().kernel_launches + (mHasHatMatrix ? 2 * (long long)mCounters.hatUpdates + 2 : 0);
     mBetas = betas;
