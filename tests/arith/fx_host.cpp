@@ -47,7 +47,7 @@ double fx_squares(const float* s, int n, double acc)
 {
     Squares q;
     for (int i = 0; i < n; i++) q.add(s[i]);
-    return q.any() ? q.add_to(acc) : acc;
+    return acc + q.sum();
 }
 
 }

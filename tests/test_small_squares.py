@@ -1,7 +1,7 @@
 """The mixed hat pass's sums of squares (csrc/fx_weight.cuh, Squares), compiled for the host, against exact sums.
 
-A square below 2^-16 is rounded to 2^-92, one above to 2^-60 of at least 2^-32, and the small ones next to a large one
-are truncated to 2^-60: 2^-27 of the sum while the largest value is above 2^-32, absolutely 8 x 2^-93 below that."""
+The bar is 2^-27 of the sum, well below the 2^-23 that the rounding of a float is of its square, for values of any
+magnitude (absolutely 8 x 2^-93 where nothing is above 2^-33); in the pass a sum spans up to 64 values, 2^-40."""
 import ctypes
 import os
 import random
@@ -34,6 +34,14 @@ def test_sums(host, low, high):
         want = sum(Fraction(float(v)) ** 2 for v in s)
         got = Fraction(host.fx_squares(s.ctypes.data, n, 0.0))
         assert abs(got - want) <= want * Fraction(1, 2 ** 27) + Fraction(8, 2 ** 93), (s, float(got), float(want))
+
+
+def test_a_pass_long(host):
+    rng = np.random.default_rng(1)
+    for low in (-1, -20, -40):
+        s = (rng.standard_normal(64) * 2.0 ** low).astype(np.float32)
+        want = sum(Fraction(float(v)) ** 2 for v in s)
+        assert abs(Fraction(host.fx_squares(s.ctypes.data, 64, 0.0)) - want) <= want * Fraction(1, 2 ** 40)
 
 
 def test_edges(host):
