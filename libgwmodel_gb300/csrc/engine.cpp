@@ -1415,15 +1415,37 @@ FxGuard Engine::fxGuard(int rows, const int* done)
     return g;
 }
 
-// The FP64 contraction over every row block, or only those that flags marks unless *all.
+// The blocks that guard_flags_ marks, for sums of up to mcols columns.
+RowBlocks Engine::guardBlocks(int mcols)
+{
+    std::vector<int> marks(guard_flags_.size()), list;
+    check(cudaMemcpyAsync(marks.data(), guard_flags_.get(), sizeof(int) * marks.size(), cudaMemcpyDeviceToHost, stream_),
+          "D2H marks");
+    synchronize();
+    for (size_t b = 0; b < marks.size(); b++)
+        if (marks[b]) list.push_back((int)b);
+    guard_list_.alloc(list.size());
+    check(cudaMemcpyAsync(guard_list_.get(), list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, stream_),
+          "H2D blocks");
+    synchronize();  // list goes away
+    RowBlocks b{};
+    b.list = guard_list_.get();
+    b.count = (int)list.size();
+    b.nsplit = contract64_splits(b.count, (n_ + kTile - 1) / kTile, num_sms_);
+    if (b.nsplit > 1) fx_part_.alloc((size_t)b.nsplit * b.count * kRowBlock * std::min(256, mcols));
+    b.part = fx_part_.get();
+    return b;
+}
+
+// The FP64 contraction over every row block, or only some of them.
 void Engine::contractRows(const double* Z, int mcols, double* G, int ldg, double bw, bool adaptive, int kernel,
-                          bool exclude_self, int wpow, const int* flags, const int* all)
+                          bool exclude_self, int wpow, const RowBlocks& blocks)
 {
     // the kernel takes at most 256 columns (p <= 21); wider Z (p up to 32) in column chunks
     for (int c0 = 0; c0 < mcols; c0 += 256) {
         const int w = std::min(256, mcols - c0);
         check(launch_contract64(points(), geographic_, tb16_.get(), Z + c0, m_, w, G + c0, ldg, thrPtr(adaptive), bw,
-                                kernel, exclude_self, wpow, true, stream_, flags, all),
+                                kernel, exclude_self, wpow, true, stream_, blocks),
               "contract64");
         stats_.kernel_launches += 1;
     }
@@ -1438,8 +1460,8 @@ void Engine::contract(const double* Z, int mcols, double* G, int ldg, double bw,
                                         exclude_self, wpow, ixy_exact_,
                                         fxLimits(bw, adaptive, kernel, wpow), use);
     if (rest)
-        contractRows(Z, mcols, G, ldg, bw, adaptive, kernel, exclude_self, wpow, fx ? fx_flags_.get() : nullptr,
-                     fx ? fx_state_.get() : nullptr);
+        contractRows(Z, mcols, G, ldg, bw, adaptive, kernel, exclude_self, wpow,
+                     fx ? RowBlocks{fx_flags_.get(), fx_state_.get(), nullptr, 0, 0, nullptr} : RowBlocks{});
     if (wpow == 1) {
         g_fx_ = fx;
         g_flagged_ = fx && rest;
@@ -1515,11 +1537,9 @@ void Engine::solve(int mode, double bw, bool adaptive, int kernel, double out[4]
     synchronize();
     if (fx) fxCheck();
     if (guarded && guard_hit_) {
-        contractRows(z_.get(), m_, g_.get(), m_, bw, adaptive, kernel, mode == kSolveCV, 1, guard_flags_.get(),
-                     fx_state_.get());
-        if (a.guard.lim2)
-            contractRows(z_.get(), mm_, g2_.get(), mm_, bw, adaptive, kernel, false, 2, guard_flags_.get(),
-                         fx_state_.get());
+        const RowBlocks marked = guardBlocks(m_);
+        contractRows(z_.get(), m_, g_.get(), m_, bw, adaptive, kernel, mode == kSolveCV, 1, marked);
+        if (a.guard.lim2) contractRows(z_.get(), mm_, g2_.get(), mm_, bw, adaptive, kernel, false, 2, marked);
         a.guard = FxGuard{};
         check(launch_solve(a, &nb, stream_), "solve");
         stats_.kernel_launches += 1;
@@ -1919,16 +1939,16 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     } else {
         fx = false;
     }
-    const auto contractFocus = [&](const int* flags) {
+    const auto contractFocus = [&](const RowBlocks& blocks) {
         for (int c0 = 0; c0 < m_; c0 += 256) {  // at most 256 columns a launch
             check(launch_contract64_focus(points(), tb16_.get(), F, pf_tb16_.get(), geographic_, z_.get() + c0, m_,
                                           std::min(256, m_ - c0), pf_g_.get() + c0, m_, thr, bw, kernel, false, 1, true,
-                                          stream_, flags, flags ? fx_state_.get() : nullptr),
+                                          stream_, blocks),
                   "predict contraction");
             stats_.kernel_launches += 1;
         }
     };
-    contractFocus(fx ? fx_flags_.get() : nullptr);
+    contractFocus(fx ? RowBlocks{fx_flags_.get(), fx_state_.get(), nullptr, 0, 0, nullptr} : RowBlocks{});
     pf_beta_.alloc((size_t)nr * p);
     SolveArgs a{};
     a.n = nr;
@@ -1966,7 +1986,7 @@ void Engine::predict(int nr, const double* locations, double bw, bool adaptive, 
     if (fx) {
         fxCheck();
         if (guard_hit_) {
-            contractFocus(guard_flags_.get());
+            contractFocus(guardBlocks(m_));
             a.guard = FxGuard{};
             solveAll();
         }

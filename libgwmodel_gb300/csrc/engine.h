@@ -347,9 +347,10 @@ private:
     FxLimits fxLimits(double bw, bool adaptive, int kernel, int wpow) const;
     DevBuf<int> refine_low_;
     void contractRows(const double* Z, int mcols, double* G, int ldg, double bw, bool adaptive, int kernel,
-                      bool exclude_self, int wpow, const int* flags, const int* all);
+                      bool exclude_self, int wpow, const RowBlocks& blocks);
+    RowBlocks guardBlocks(int mcols);
     DevBuf<double> zfx_sum_, fx_lim_;  // fx_lim_: limits of G, then of G2
-    DevBuf<int> guard_flags_;
+    DevBuf<int> guard_flags_, guard_list_;
     int guard_hit_ = 0;                  // guard_flags_ marks rows of the last guarded solve (FxGuard::any)
     bool g_fx_ = false, g2_fx_ = false;  // g_, g2_ hold fixed-point sums
     bool g_flagged_ = false;             // ... whose blocks in fx_flags_ k_contract64 has recomputed

@@ -109,19 +109,27 @@ cudaError_t launch_build_z(int n, int p, const double* X, const double* y, doubl
 // (r_i = thr[i], or bw when thr is null); exclude_self zeroes w_ii (CV).
 // FP64 SIMT, the weight matrix is produced tile by tile and never stored.
 // tb16: FP32 bounds of the 16-point tiles (planar box or geographic cap).
-// flags (optional): only the 64-row blocks with a nonzero flag are computed, or
-// every block when *all is nonzero.
+// blocks (optional): only some of the 64-row blocks.
+struct RowBlocks {
+    const int *flags, *all;  // those with a nonzero flag, or every one when *all is nonzero
+    // or an ordered list of them, whose tiles are split nsplit ways where that many blocks
+    // leave SMs idle (part: nsplit x count x 64 x mcols doubles of scratch)
+    const int* list;
+    int count, nsplit;
+    double* part;
+};
 cudaError_t launch_contract64(const DevPoints& P, bool geographic, const float4* tb16, const double* Z, int ldz,
                               int mcols, double* G, int ldg, const double* thr, double bw, int kernel,
                               bool exclude_self, int wpow, bool skip_tiles, cudaStream_t stream,
-                              const int* flags = nullptr, const int* all = nullptr);
+                              const RowBlocks& blocks = RowBlocks{});
 // The same with focus rows F (their 16-point tile bounds ftb16) that are not
 // the data points: G[i, :] for every focus row i over the data P (predict).
 cudaError_t launch_contract64_focus(const DevPoints& P, const float4* tb16, const DevPoints& F, const float4* ftb16,
                                     bool geographic, const double* Z, int ldz, int mcols, double* G, int ldg,
                                     const double* thr, double bw, int kernel, bool exclude_self, int wpow,
-                                    bool skip_tiles, cudaStream_t stream, const int* flags = nullptr,
-                                    const int* all = nullptr);
+                                    bool skip_tiles, cudaStream_t stream, const RowBlocks& blocks = RowBlocks{});
+// Splits of the tiles for `count` row blocks.
+int contract64_splits(int count, int ntiles, int num_sms);
 
 // Which rows of fixed-point sums are less exact than FP64 ones because a column of X
 // rests on small weights there (a covariate that is zero near the row's location): the

@@ -11,6 +11,8 @@
 //
 // GB300 runs FP64 at a small fraction of its FP32/tensor rate, so this
 // kernel is bound by the FP64 pipe; its job is to be the exact drop-in.
+#include <algorithm>
+
 #include "gw_common.cuh"
 #include "gw_kernels.h"
 #include "pair_weight64.cuh"
@@ -24,15 +26,45 @@ constexpr int CT_BM = kRowBlock;  // 64 focus rows
 constexpr int CT_BK = kTile;      // 16 data points per tile
 constexpr int CT_ROWS_PER_THREAD = CT_BM / 16;
 
+// First tile of a split (blockIdx.y).
+__device__ __forceinline__ int split_tile(int ntiles, int split)
+{
+    return (int)((long long)ntiles * split / gridDim.y);
+}
+
+// Where a CTA's rows go: to G, or to its split's part.
+struct RowsOut {
+    double* at;
+    int ld;
+};
+__device__ __forceinline__ RowsOut rows_out(const RowBlocks& b, double* G, int ldg, int mcols, int row0)
+{
+    if (gridDim.y == 1) return RowsOut{G + (size_t)row0 * ldg, ldg};
+    return RowsOut{b.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * CT_BM * mcols, mcols};
+}
+
+// G's rows of the listed blocks: the splits' sums in order.
+__global__ void k_rows_finish(RowBlocks b, int nf, int mcols, double* __restrict__ G, int ldg)
+{
+    const int row0 = b.list[blockIdx.x] * CT_BM, rows = min(CT_BM, nf - row0);
+    const size_t stride = (size_t)b.count * CT_BM * mcols;
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < rows * mcols; e += gridDim.y * blockDim.x) {
+        const double* p = b.part + (size_t)blockIdx.x * CT_BM * mcols + e;
+        double v = 0.0;
+        for (int s = 0; s < b.nsplit; s++) v += p[s * stride];
+        G[(size_t)(row0 + e / mcols) * ldg + e % mcols] = v;
+    }
+}
+
 template <bool GEO, int NC>
 __global__ void __launch_bounds__(CT_THREADS)
     k_contract64(DevPoints P, const float4* __restrict__ tb16, DevPoints F, const float4* __restrict__ ftb16,
                  const double* __restrict__ Z, int ldz, int mcols, double* __restrict__ G, int ldg,
                  const double* __restrict__ thr, double bw, int kernel, int exclude_self, int wpow, int skip_tiles,
-                 const int* __restrict__ flags, const int* __restrict__ all)
+                 RowBlocks blocks)
 {
     constexpr int NCOL = NC * 16;
-    if (flags && !flags[blockIdx.x] && !*all) return;
+    if (blocks.flags && !blocks.flags[blockIdx.x] && !*blocks.all) return;
     __shared__ double sW[CT_BM][CT_BK + 1];
     __shared__ double sZ[CT_BK][NCOL];
     __shared__ double sfu[CT_BM], sfv[CT_BM], sfuR[CT_BM], sfvR[CT_BM], sthr[CT_BM], sr2[CT_BM], sir2[CT_BM];
@@ -42,7 +74,7 @@ __global__ void __launch_bounds__(CT_THREADS)
 
     const int n = P.n, nf = F.n;  // data points, focus rows (the data themselves, or prediction points)
     const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const int row0 = blockIdx.x * CT_BM;
+    const int row0 = (blocks.list ? blocks.list[blockIdx.x] : (int)blockIdx.x) * CT_BM;
     // unit-vector distances for geographic data unless the boxcar step needs the reference formula
     const bool vec = GEO && P.e && F.e && kernel != GW_KERNEL_BOXCAR;
 
@@ -76,6 +108,9 @@ __global__ void __launch_bounds__(CT_THREADS)
     const float4 fbound = sbound;
     const float far_thr = (skip_tiles && kernel >= GW_KERNEL_BISQUARE) ? tb_far_threshold<GEO>(rmax) : -1.0f;
 
+    // (row0 and nf, which the loop needs no more, take fewer registers this way)
+    const int rows = min(CT_BM, nf - row0), self0 = exclude_self ? row0 : -CT_BM;
+
     double acc[CT_ROWS_PER_THREAD][NC];
 #pragma unroll
     for (int q = 0; q < CT_ROWS_PER_THREAD; q++)
@@ -83,7 +118,8 @@ __global__ void __launch_bounds__(CT_THREADS)
         for (int c = 0; c < NC; c++) acc[q][c] = 0.0;
 
     const int ntiles = (n + CT_BK - 1) / CT_BK;
-    for (int tile = 0; tile < ntiles; tile++) {
+    const int end = split_tile(ntiles, blockIdx.y + 1);
+    for (int tile = split_tile(ntiles, blockIdx.y); tile < end; tile++) {
         if (tb_far<GEO>(fbound, tb16[tile], far_thr)) continue;  // uniform over the CTA
         const int j0 = tile * CT_BK;
         // Z tile -> shared (zero padded)
@@ -105,13 +141,12 @@ __global__ void __launch_bounds__(CT_THREADS)
 #pragma unroll
             for (int q = 0; q < CT_ROWS_PER_THREAD; q++) {
                 const int r = ty + 16 * q;
-                const int i = row0 + r;
                 double w = 0.0;
-                if (j < n && i < nf) {
+                if (j < n && r < rows) {
                     w = vec ? pair_weight64_vec(kernel, sfe[0][r], sfe[1][r], sfe[2][r], ex, ey, ez, sthr[r], sir2[r])
                             : pair_weight64<GEO>(kernel, du, dv, duR, dvR, sfu[r], sfv[r], sfuR[r], sfvR[r], sthr[r],
                                                  sr2[r], sir2[r]);
-                    if (exclude_self && i == j) w = 0.0;
+                    if (r == j - self0) w = 0.0;
                     if (wpow == 2) w = w * w;
                 }
                 sW[r][tx] = w;
@@ -132,14 +167,15 @@ __global__ void __launch_bounds__(CT_THREADS)
         }
         __syncthreads();
     }
+    const RowsOut out = rows_out(blocks, G, ldg, mcols, row0);
 #pragma unroll
     for (int q = 0; q < CT_ROWS_PER_THREAD; q++) {
-        const int i = row0 + ty + 16 * q;
-        if (i >= nf) continue;
+        const int r = ty + 16 * q;
+        if (r >= rows) continue;
 #pragma unroll
         for (int c = 0; c < NC; c++) {
             const int col = tx + 16 * c;
-            if (col < mcols) G[(size_t)i * ldg + col] = acc[q][c];
+            if (col < mcols) out.at[(size_t)r * out.ld + col] = acc[q][c];
         }
     }
 }
@@ -154,10 +190,10 @@ __global__ void __launch_bounds__(CT_THREADS)
     k_contract64_narrow(DevPoints P, const float4* __restrict__ tb16, DevPoints F, const float4* __restrict__ ftb16,
                         const double* __restrict__ Z, int ldz, double* __restrict__ G, int ldg,
                         const double* __restrict__ thr, double bw, int kernel, int exclude_self, int wpow,
-                        int skip_tiles, const int* __restrict__ flags, const int* __restrict__ all)
+                        int skip_tiles, RowBlocks blocks)
 {
     constexpr int BM = 16 * RPT;  // rows of this CTA
-    if (flags && !flags[blockIdx.x * BM / CT_BM] && !*all) return;
+    if (blocks.flags && !blocks.flags[blockIdx.x * BM / CT_BM] && !*blocks.all) return;
     __shared__ double sfu[BM], sfv[BM], sfuR[BM], sfvR[BM], sthr[BM], sr2[BM], sir2[BM];
     __shared__ double sfe[3][BM];
     __shared__ double sred[CT_THREADS / 32];
@@ -165,7 +201,7 @@ __global__ void __launch_bounds__(CT_THREADS)
 
     const int n = P.n, nf = F.n;
     const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const int row0 = blockIdx.x * BM;
+    const int row0 = (blocks.list ? blocks.list[blockIdx.x] : (int)blockIdx.x) * BM;  // (a list: BM is 64)
     const bool vec = GEO && P.e && F.e && kernel != GW_KERNEL_BOXCAR;
 
     double rmax = bw;
@@ -222,7 +258,8 @@ __global__ void __launch_bounds__(CT_THREADS)
         for (int c = 0; c < M; c++) acc[q][c] = 0.0;
 
     const int ntiles = (n + CT_BK - 1) / CT_BK;
-    for (int tile = 0; tile < ntiles; tile++) {
+    const int end = split_tile(ntiles, blockIdx.y + 1);
+    for (int tile = split_tile(ntiles, blockIdx.y); tile < end; tile++) {
         if (tb_far<GEO>(fbound, tb16[tile], far_thr)) continue;  // uniform over the CTA
         const int j = tile * CT_BK + tx;
         if (j >= n) continue;
@@ -245,6 +282,7 @@ __global__ void __launch_bounds__(CT_THREADS)
             for (int c = 0; c < M; c++) acc[q][c] = fma(w, z[c], acc[q][c]);
         }
     }
+    const RowsOut out = rows_out(blocks, G, ldg, M, row0);
 #pragma unroll
     for (int q = 0; q < RPT; q++)
 #pragma unroll
@@ -252,36 +290,34 @@ __global__ void __launch_bounds__(CT_THREADS)
             double v = acc[q][c];
 #pragma unroll
             for (int off = 8; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            if (tx == 0 && ri[q] >= 0) G[(size_t)ri[q] * ldg + c] = v;
+            if (tx == 0 && ri[q] >= 0) out.at[(size_t)(ri[q] - row0) * out.ld + c] = v;
         }
 }
 
 template <bool GEO, int NC>
 cudaError_t launch_nc(const DevPoints& P, const float4* tiles, const DevPoints& F, const float4* ftiles,
                       const double* Z, int ldz, int mcols, double* G, int ldg, const double* thr, double bw,
-                      int kernel, bool exclude_self, int wpow, bool skip, cudaStream_t s, const int* flags,
-                      const int* all)
+                      int kernel, bool exclude_self, int wpow, bool skip, cudaStream_t s, const RowBlocks& b)
 {
-    int grid = (F.n + CT_BM - 1) / CT_BM;
+    const dim3 grid(b.list ? b.count : (F.n + CT_BM - 1) / CT_BM, b.list ? b.nsplit : 1);
     k_contract64<GEO, NC><<<grid, CT_THREADS, 0, s>>>(P, tiles, F, ftiles, Z, ldz, mcols, G, ldg, thr, bw, kernel,
-                                                     exclude_self ? 1 : 0, wpow, skip ? 1 : 0, flags, all);
+                                                     exclude_self ? 1 : 0, wpow, skip ? 1 : 0, b);
     return cudaGetLastError();
 }
 
 template <bool GEO>
 cudaError_t launch_geo(const DevPoints& P, const float4* tiles, const DevPoints& F, const float4* ftiles,
                        const double* Z, int ldz, int mcols, double* G, int ldg, const double* thr, double bw,
-                       int kernel, bool exclude_self, int wpow, bool skip, cudaStream_t s, const int* flags,
-                      const int* all)
+                       int kernel, bool exclude_self, int wpow, bool skip, cudaStream_t s, const RowBlocks& b)
 {
     if (mcols <= 4) {
-        // rows per CTA: 64 when that already gives a few CTAs per SM, else 32 or 16
-        const int rpt = F.n >= 64 * 152 * 4 ? 4 : (F.n >= 32 * 152 * 4 ? 2 : 1);
-        const int grid = (F.n + 16 * rpt - 1) / (16 * rpt);
+        // rows per CTA: 64 when that already gives a few CTAs per SM (or the blocks are split), else 32 or 16
+        const int rpt = b.list || F.n >= 64 * 152 * 4 ? 4 : (F.n >= 32 * 152 * 4 ? 2 : 1);
+        const dim3 grid(b.list ? b.count : (F.n + 16 * rpt - 1) / (16 * rpt), b.list ? b.nsplit : 1);
         const int ex = exclude_self ? 1 : 0, sk = skip ? 1 : 0;
 #define GW_NARROW(MM, R)                                                                                        \
     k_contract64_narrow<GEO, MM, R><<<grid, CT_THREADS, 0, s>>>(P, tiles, F, ftiles, Z, ldz, G, ldg, thr, bw, \
-                                                                kernel, ex, wpow, sk, flags, all)
+                                                                kernel, ex, wpow, sk, b)
 #define GW_NARROW_M(MM)            \
     if (rpt == 4)                  \
         GW_NARROW(MM, 4);          \
@@ -303,7 +339,7 @@ cudaError_t launch_geo(const DevPoints& P, const float4* tiles, const DevPoints&
 #define GW_NC_CASE(K) \
     case K:           \
         return launch_nc<GEO, K>(P, tiles, F, ftiles, Z, ldz, mcols, G, ldg, thr, bw, kernel, exclude_self, wpow, \
-                                 skip, s, flags, all);
+                                 skip, s, b);
     switch (nc) {
         GW_NC_CASE(1) GW_NC_CASE(2) GW_NC_CASE(3) GW_NC_CASE(4) GW_NC_CASE(5) GW_NC_CASE(6) GW_NC_CASE(7)
         GW_NC_CASE(8) GW_NC_CASE(9) GW_NC_CASE(10) GW_NC_CASE(11) GW_NC_CASE(12) GW_NC_CASE(13)
@@ -317,24 +353,33 @@ cudaError_t launch_geo(const DevPoints& P, const float4* tiles, const DevPoints&
 
 cudaError_t launch_contract64(const DevPoints& P, bool geographic, const float4* tb16, const double* Z, int ldz,
                               int mcols, double* G, int ldg, const double* thr, double bw, int kernel,
-                              bool exclude_self, int wpow, bool skip_tiles, cudaStream_t stream, const int* flags,
-                              const int* all)
+                              bool exclude_self, int wpow, bool skip_tiles, cudaStream_t stream, const RowBlocks& blocks)
 {
     return launch_contract64_focus(P, tb16, P, tb16, geographic, Z, ldz, mcols, G, ldg, thr, bw, kernel, exclude_self,
-                                   wpow, skip_tiles, stream, flags, all);
+                                   wpow, skip_tiles, stream, blocks);
 }
 
 cudaError_t launch_contract64_focus(const DevPoints& P, const float4* tb16, const DevPoints& F, const float4* ftb16,
                                     bool geographic, const double* Z, int ldz, int mcols, double* G, int ldg,
                                     const double* thr, double bw, int kernel, bool exclude_self, int wpow,
-                                    bool skip_tiles, cudaStream_t stream, const int* flags, const int* all)
+                                    bool skip_tiles, cudaStream_t stream, const RowBlocks& blocks)
 {
     if (mcols < 1 || mcols > 256 || F.n < 1) return cudaErrorInvalidValue;
-    if (geographic)
-        return launch_geo<true>(P, tb16, F, ftb16, Z, ldz, mcols, G, ldg, thr, bw, kernel, exclude_self, wpow,
-                                skip_tiles, stream, flags, all);
-    return launch_geo<false>(P, tb16, F, ftb16, Z, ldz, mcols, G, ldg, thr, bw, kernel, exclude_self, wpow,
-                             skip_tiles, stream, flags, all);
+    const cudaError_t rc =
+        geographic ? launch_geo<true>(P, tb16, F, ftb16, Z, ldz, mcols, G, ldg, thr, bw, kernel, exclude_self, wpow,
+                                      skip_tiles, stream, blocks)
+                   : launch_geo<false>(P, tb16, F, ftb16, Z, ldz, mcols, G, ldg, thr, bw, kernel, exclude_self, wpow,
+                                       skip_tiles, stream, blocks);
+    if (rc != cudaSuccess || !blocks.list || blocks.nsplit == 1) return rc;
+    k_rows_finish<<<dim3(blocks.count, 4), 256, 0, stream>>>(blocks, F.n, mcols, G, ldg);
+    return cudaGetLastError();
+}
+
+// Four CTAs per SM, which also evens out blocks that fall on the SMs unequally; a split
+// keeps 8 tiles.
+int contract64_splits(int count, int ntiles, int num_sms)
+{
+    return std::max(1, std::min(std::min(ntiles / 8, 16), (4 * num_sms + count - 1) / count));
 }
 
 }  // namespace gwgpu

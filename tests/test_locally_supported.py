@@ -68,6 +68,20 @@ def test_bisquare_rows_that_reach_the_region_with_their_rim(geographic):
     check(e, ref, bw, False, O.BISQUARE)
 
 
+@pytest.mark.parametrize("n,p,bw", [(3001, 3, 12.0), (1100, 1, 3.0), (2049, 11, 16.0)])
+def test_some_blocks_of_many(n, p, bw):
+    """Marked blocks are recomputed from a list, their tiles split: partial blocks and tiles, column counts of the
+    narrow form (p = 1: an uncentred column alone) and of several groups, rows marked in one region only."""
+    x, y, c = problem(n, 7, False)
+    rng = np.random.default_rng(p)
+    if p == 1:  # small where it is not 1, so that no system is singular
+        x = np.asfortranarray(np.where(x[:, 2:] > 0, 1.0, 1e-2 * (1.0 + rng.random((n, 1)))))
+        y = x[:, 0] + rng.normal(0, 0.1, n)
+    else:
+        x = np.asfortranarray(np.column_stack([x, rng.standard_normal((n, p - 3))]))
+    check(engine(x, y, c, False), O.Problem(x, y, c), bw, False, O.GAUSSIAN, c[::11] + 0.01)
+
+
 @pytest.mark.parametrize("p", [11, 24])
 def test_indicator_among_many_columns(p):
     """Column groups after the first and the warp form of the solve (p > 20)."""
