@@ -10,7 +10,9 @@
 // than the largest threshold of the CTA's 64 rows (planar coordinates).
 //
 // GB300 runs FP64 at a small fraction of its FP32/tensor rate, so this
-// kernel is bound by the FP64 pipe; its job is to be the exact drop-in.
+// kernel is bound by the FP64 pipe; its job is to be the exact drop-in, for the
+// kernels without a fixed-point form and for the rows that k_contract_fx's sums do
+// not hold exactly enough (RowBlocks).
 #include <algorithm>
 
 #include "gw_common.cuh"
@@ -376,7 +378,8 @@ cudaError_t launch_contract64_focus(const DevPoints& P, const float4* tb16, cons
 }
 
 // Four CTAs per SM, which also evens out blocks that fall on the SMs unequally; a split
-// keeps 8 tiles.
+// keeps 8 tiles.  An evaluation whose blocks are all marked: n = 600 0.52 -> 0.24 ms, n = 5,000
+// 3.7 -> 1.7, n = 20,000 41.9 -> 22.2 against one CTA a block wherever it lay.
 int contract64_splits(int count, int ntiles, int num_sms)
 {
     return std::max(1, std::min(std::min(ntiles / 8, 16), (4 * num_sms + count - 1) / count));
