@@ -1786,7 +1786,10 @@ size_t Engine::estimateBytes(int n, int p, bool geographic, bool mixed, bool ada
             splits = std::max(splits, fx_splits((n + 127) / 128 * g, (n + 15) / 16, num_sms));
         b += 40 * N + 8 * N * hat_splits(n, num_sms);
         b += t16 * groups * w * 256 + std::ceil(N / 1024) * groups * w * 20 + 32 * N;
-        b += (splits > 1 ? 8 * N * m * splits : 0.0) + 4 * N * splits + N;
+        // their splits' sums, or those of the blocks that FP64 sums replace (contract64_splits)
+        const double blocks = std::ceil(N / kRowBlock), ctas = std::min(16 * blocks, 4.0 * num_sms + std::min(blocks, 4.0 * num_sms));
+        const double marked = 8.0 * kRowBlock * std::min(256.0, m) * ctas;
+        b += std::max(splits > 1 ? 8 * N * m * splits : 0.0, marked) + 4 * N * splits + N;
     }
     if (adaptive) {
         const double h = 4.0 * (4096 + 64) * N;  // histograms and their segment counts
