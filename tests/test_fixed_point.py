@@ -315,3 +315,20 @@ def test_timeout_is_reported_and_engine_recovers(n, p, geographic, kernel):
             f()
         e.set_tc_wait_limit(0)
         assert np.array_equal(f(), w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("geographic", [False, True])
+@pytest.mark.parametrize("n,kernel", [(129, O.BISQUARE), (129, O.GAUSSIAN), (701, O.BISQUARE), (701, O.GAUSSIAN)])
+def test_hat_matrix_entries(n, kernel, geographic):
+    """S whole, and its last row where it is not stored (fixed-point weights there): 1e-9 of the largest entry."""
+    x, y, coords = problem(n, 4, n)
+    g = degrees(coords, 5.0, 45.0, 10.0) if geographic else coords
+    e, ref = engine(x, y, g, geographic), O.Problem(x, y, g, geographic=geographic)
+    want = ref.fit_core(n // 2, True, kernel)
+    for store in (True, False):
+        got = e.fit(n // 2, True, kernel, store)
+        S = want[4] if store else ref.fit_core(n // 2, True, kernel, False)[4]
+        assert got[4].shape == S.shape
+        assert np.abs(got[4] - S).max() <= 1e-9 * np.abs(S).max()
+        np.testing.assert_allclose(got[3], want[3], rtol=1e-9)

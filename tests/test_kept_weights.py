@@ -1,4 +1,5 @@
 """Weights kept between the passes of a call: one buffer per device for all engines on it, given back with the last."""
+import gc
 import threading
 
 import numpy as np
@@ -26,6 +27,7 @@ def fitted(n, p, seed):
 def test_one_buffer_for_two_engines_and_none_after_them():
     torch = pytest.importorskip("torch")
     torch.cuda.init()
+    gc.collect()  # no engine of an earlier test
     n, p = 20011, 12
     free = lambda: torch.cuda.mem_get_info(0)[0]
     warm = Engine(0)
